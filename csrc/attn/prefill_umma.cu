@@ -1,5 +1,6 @@
 // Prefill attention on the 5th-generation tensor cores: variable-length, causal, GQA, keys and values read from
-// the paged cache (tinyvllm/layers/attention.py:99-105 calls flash_attn_varlen_func).
+// the paged cache (tinyvllm/layers/attention.py:99-105 calls flash_attn_varlen_func).  One query tile per CTA: for batches whose tiles all
+// run at once; prefill_pair.cu has the kernel for more of them, and the rule is in forge_prefill_attention_umma.
 //
 // CTA = 128 query rows of one (sequence, q head); KV tiles of 128 keys (one tile never straddles a cache block:
 // block_size >= 128).  Both products run as tcgen05.mma with fp32 accumulators in tensor memory:
@@ -23,6 +24,8 @@
 #include "../include/launch.cuh"
 #include "../include/ptx.cuh"
 
+#include <algorithm>
+
 namespace forge {
 
 constexpr int kUD = 128;                  // head_dim
@@ -32,19 +35,6 @@ constexpr int kUHalf = 128 * 128;         // bytes of one swizzled box: 128 rows
 constexpr int kUTile = 2 * kUHalf;        // one 128 x 128 bf16 operand
 constexpr int kUThreads = 192;
 constexpr int kUStages = 2;
-
-// Shared-memory descriptor of an MN-major operand as TMA lays it down with the 128-byte swizzle: rows are the K
-// index (keys), each row holds 64 contiguous elements of the MN index (head_dim).  Stride between 8-row groups along
-// K: 1024 bytes; stride between the two 64-element blocks along MN: one box.
-__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t mn_block_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((mn_block_bytes >> 4) & 0x3FFFu) << 16;   // leading byte offset: next 64 elements along MN
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;                         // stride byte offset: next 8 rows along K
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;                                 // SWIZZLE_128B
-  return d;
-}
 
 // Row maximum of the raw scores of one tile; kMasked: only keys kbase + i < limit count.  Four chains, not one.
 template <bool kMasked>
@@ -324,6 +314,10 @@ __global__ void __launch_bounds__(kUThreads, 1) prefill_attn_umma_kernel(
   }
 }
 
+int launch_prefill_attn_pair(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const int* cu_q, const int* lens,
+                             const int* bt, void* out, int T, int num_seqs, int max_q, int nq, int nkv, int block_size, int table_width,
+                             int num_blocks, float scale_log2, unsigned* status, cudaStream_t stream);
+
 extern "C" int forge_make_tmap_2d(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                                   uint32_t box_rows, int elem_bytes);
 
@@ -339,12 +333,20 @@ extern "C" int forge_prefill_attention_umma(const void* q, const void* kc, const
   const uint64_t rows = static_cast<uint64_t>(num_blocks) * nkv * block_size;
   if (forge_make_tmap_2d(&tm_k, kc, rows, kUD, kUD, kUN, 2) != 0) return -2;
   if (forge_make_tmap_2d(&tm_v, vc, rows, kUD, kUD, kUN, 2) != 0) return -2;
+  const float scale_log2 = scale * 1.4426950408889634f;
+  // One tile per CTA while all tiles run at once: alone, a tile's chain over the keys is shorter than next to another one.  From then on two per
+  // CTA (prefill_pair.cu).  Measured, one against two: 1 x 1000 tokens of 16 heads (128 tiles) 22.6 / 31.7 us, 4 x 700 of 5 heads (120) 20.5 / 25.6;
+  // 12 x 100 of 16 heads (192) 20.6 / 16.4, 1 x 700 of 32 heads (192) 28.7 / 24.6, 1 x 1300 of 16 heads (176) 35.6 / 35.6, 2 x 513 of 32 heads 34.8 / 24.6.
+  const long long tiles = std::min<long long>(static_cast<long long>(num_seqs) * ((max_q + kUM - 1) / kUM), T / kUM + num_seqs) * nq;
+  if (tiles > device_sm_count())
+    return launch_prefill_attn_pair(tm_q, tm_k, tm_v, cu_q, lens, bt, out, T, num_seqs, max_q, nq, nkv, block_size, table_width, num_blocks, scale_log2,
+                                    status, stream);
   constexpr int smem = (1 + 2 * kUStages + 2) * kUTile + 256 + 1024;
   FORGE_ENSURE_DYN_SMEM(prefill_attn_umma_kernel, smem);
   dim3 grid((max_q + kUM - 1) / kUM, nq, num_seqs);
   return launch_kernel(prefill_attn_umma_kernel, grid, dim3(kUThreads), smem, stream, 0, tm_q, tm_k, tm_v, cu_q, lens, bt,
                        static_cast<__nv_bfloat16*>(out), nq, nkv, block_size, table_width, num_blocks,
-                       scale * 1.4426950408889634f, status) == cudaSuccess ? 0 : -5;
+                       scale_log2, status) == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace forge

@@ -71,6 +71,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// One look, without a wait.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait. ~4M polls; each try_wait may itself suspend for a short, hardware-chosen time.
 constexpr uint32_t kMbarSpinLimit = 1u << 22;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned* status) {
@@ -169,6 +181,19 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
   d |= static_cast<uint64_t>(1024 >> 4) << 32;                     // stride byte offset: 8 rows * 128 B
   d |= static_cast<uint64_t>(1) << 46;                             // descriptor version (Blackwell)
   d |= static_cast<uint64_t>(2) << 61;                             // SWIZZLE_128B
+  return d;
+}
+
+// Shared-memory descriptor of an MN-major operand as TMA lays it down with the 128-byte swizzle: rows are the K
+// index (keys), each row holds 64 contiguous elements of the MN index (head_dim).  Stride between 8-row groups along
+// K: 1024 bytes; stride between the two 64-element blocks along MN: one box.
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t mn_block_bytes) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>((mn_block_bytes >> 4) & 0x3FFFu) << 16;   // leading byte offset: next 64 elements along MN
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;                         // stride byte offset: next 8 rows along K
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(2) << 61;                                 // SWIZZLE_128B
   return d;
 }
 

@@ -616,6 +616,26 @@ def test_prefill_attention(ops, q_lens, k_lens, nq, nkv, bs):
     ops.check_status()
 
 
+@pytest.mark.parametrize("q_lens,k_lens,nq,nkv,bs", [
+    ([130] * 9 + [1, 127, 128, 129, 256, 257], [130] * 9 + [1, 127, 128, 129, 256, 257], 16, 8, 256),
+    ([1000, 3, 700], [1000, 3, 700], 32, 8, 256),                                # few sequences, several rounds of items per CTA
+    ([5 + 3 * i for i in range(70)], [5 + 3 * i + 128 * (i % 3) for i in range(70)], 4, 2, 128),      # three ballots of sequences, prefixes
+    ([300, 0, 129, 640, 0, 1, 511], [300, 0, 1153, 700, 256, 2, 511], 12, 4, 256),          # odd group: row pairs, with and without a second tile; empty ones
+    ([257] * 20, [257] * 20, 5, 5, 512),
+    ([256] * 3 + [64] * 9, [2304] * 3 + [2112] * 9, 32, 8, 256),                 # a prefix shared in length
+])
+def test_prefill_attention_two_tiles_per_cta(ops, q_lens, k_lens, nq, nkv, bs):
+    """More tiles than SMs: items of two heads or two row tiles, dealt out over persistent CTAs (tolerance of the test above: bf16 operands and weights)."""
+    assert sum(-(-n // 128) for n in q_lens) * nq > torch.cuda.get_device_properties(0).multi_processor_count
+    q, kc, vc, b = _paged_case(q_lens, k_lens, nq, nkv, bs, seed=2)
+    b.is_prefill = True
+    want = ref.attention(q, kc, vc, b.cu_seqlens_q, b.context_lens, b.block_tables, 128 ** -0.5, b.num_seqs)
+    for _ in range(2):
+        got = ops.attention(q, kc, vc, b, 128 ** -0.5)
+        _close(got, want, 2e-2, 2e-2)
+    ops.check_status()
+
+
 # ----------------------------------------------------------------------------- sampler
 def _header(step, seed):
     h = torch.zeros(16, dtype=torch.int32)
