@@ -1,0 +1,336 @@
+// Decode attention in context chunks on the tensor cores: few sequences, all query heads of a KV head at once.
+//
+// The work is the list of live chunks (`chunk` tokens of one sequence) times KV heads, dealt out in turn to persistent CTAs; lengths are
+// read on the device, so the launch fits a CUDA graph whatever they become.  A CTA streams tiles of 64 tokens of K and V (2-D TMA boxes
+// of 64 rows x 64 dims with the 128-byte swizzle, a ring of two stages that never drains across items) and its four consumer warps take
+// 16 tokens of each tile: S = Q K^T and O += P V as mma.sync m16n8k16 with fp32 sums.  The heads of the group fill rows 0..7 of the
+// query tile.  The weights keep 16 bits of their mantissa: P = hi + lo, two bf16 numbers; hi fills rows 0..7 of the second product
+// and lo rows 8..15, which would be empty.  A sequence of one chunk is finished here, others leave partials for the merge kernel.
+//
+// What bounds it is latency (length -> block table -> keys -> scores -> sums), and from about ten sequences the stream of the cache: three
+// CTAs per SM with 64 KB on their way each.  The dot products on the CUDA cores, which this replaces for cache blocks of 64 tokens and more,
+// took longer than the stream: a tile of 64 tokens of four heads needs 64 K multiply-adds and 2500 shuffles in a warp.
+// Measured with the merge, 32 / 8 heads (CUDA cores): 1 x 3001 tokens 24.2 -> 13.3 us, 8 x 200 .. 2000: 21.0 -> 17.8, 13: 31.7 -> 22.4, 24: 54.5 -> 39.8;
+// 64 / 8 heads, 24 x 200 .. 2000: 91 -> 36 us.  The error against 64 bits is the same (1.9e-3, the rounding of the result to bf16).
+#include <algorithm>
+
+#include "../include/decode_common.cuh"
+#include "../include/launch.cuh"
+#include "../include/mma_sync.cuh"
+#include "../include/ptx.cuh"
+
+namespace forge {
+
+constexpr int kCkTile = 64;
+constexpr int kCkBox = kCkTile * 128;                 // one TMA box: 64 token rows x 64 dims
+constexpr int kCkTileBytes = 2 * kCkBox;              // K (or V) of a tile: dims 0..63, then dims 64..127
+constexpr int kCkStages = 2;
+__host__ __device__ constexpr int ck_ctas_per_sm(int G) { return G > 4 ? 2 : 3; }
+
+// Shared-memory address of the 16-byte piece `piece` (0..15: eight dims each) of token row `r` of a swizzled tile.
+__device__ __forceinline__ uint32_t ck_addr(uint32_t tile, int r, int piece) {
+  return tile + (piece >> 3) * kCkBox + r * 128 + (((piece & 7) ^ (r & 7)) << 4);
+}
+
+struct ChunkItem {
+  int b, c, kvh, len, chunk;
+};
+
+__device__ __forceinline__ int chunk_checked_len(const int* __restrict__ lens, int b, int cap, unsigned* status) {
+  int len = lens[b];
+  if (len > cap) {                                       // a corrupted length: clamped and reported
+    set_status(status, kStatusBadIndex);
+    len = cap;
+  }
+  return max(len, 0);
+}
+
+// Item `item`; executed by whole warps.  Direct: of the list [chunk][sequence][KV head] with `parts` chunks for every sequence, dead ones have
+// c * chunk >= len.  Else of the list [live chunk][KV head].  False: there are not that many.
+__device__ __forceinline__ bool chunk_item(const int* __restrict__ lens, int B, int nkv, int unit, int parts, int cap, bool direct, int item,
+                                           unsigned* status, ChunkItem& it) {
+  const int lane = threadIdx.x & 31;
+  int left = item / nkv;
+  it.kvh = item - left * nkv;
+  if (direct) {
+    it.c = left / B;
+    it.b = left - it.c * B;
+    if (it.c >= parts) return false;
+    it.len = chunk_checked_len(lens, it.b, cap, status);
+    it.chunk = decode_chunk_tokens(it.len, unit, parts);
+    return true;
+  }
+  for (int b0 = 0; b0 < B; b0 += 32) {
+    const int len = b0 + lane < B ? chunk_checked_len(lens, b0 + lane, cap, status) : 0;
+    const int chunk = decode_chunk_tokens(len, unit, parts), n = (len + chunk - 1) / chunk;
+    int sum = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += u;
+    }
+    const uint32_t above = __ballot_sync(0xffffffffu, left < sum);
+    if (above != 0) {
+      const int l = __ffs(above) - 1;
+      it.b = b0 + l;
+      it.len = __shfl_sync(0xffffffffu, len, l);
+      it.chunk = __shfl_sync(0xffffffffu, chunk, l);
+      it.c = left - __shfl_sync(0xffffffffu, sum - n, l);
+      return true;
+    }
+    left -= __shfl_sync(0xffffffffu, sum, 31);
+  }
+  return false;
+}
+
+template <int G>
+__global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_chunk_kernel(
+    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __nv_bfloat16* __restrict__ q,
+    __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, const int* __restrict__ block_tables, const int* __restrict__ context_lens,
+    __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml, int B, int nq, int nkv, int block_size,
+    int table_width, int num_blocks, int unit, int max_chunks, int parts, int direct, float scale_log2, unsigned* status, const DecodeFuse fuse) {
+  static_assert(G <= 8, "the heads of a group fill the first eight rows of the query tile");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  float* s_acc = reinterpret_cast<float*>(smem + kCkStages * 2 * kCkTileBytes);          // merge area
+  __nv_bfloat16* s_q = reinterpret_cast<__nv_bfloat16*>(s_acc + decode_merge_floats(G)); // [G][128]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(s_q + G * kD);
+  uint64_t* empty_bar = full_bar + kCkStages;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cap = min(table_width * block_size, max_chunks * unit);
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&tm_k);
+    prefetch_tensormap(&tm_v);
+    for (int s = 0; s < kCkStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 4);
+    }
+    fence_mbar_init();
+  }
+  __syncthreads();
+  pdl_wait();                                           // q, the cache and the step buffer come from predecessors
+
+  ChunkItem it;
+  if (warp == 4) {
+    // ------------------------------------------------------------------ producer
+    int n = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; ok && chunk_item(context_lens, B, nkv, unit, parts, cap, direct != 0, item, status, it); item += gridDim.x) {
+      if (lane == 0) {
+        const int end = min(it.len, (it.c + 1) * it.chunk);
+        for (int tok = it.c * it.chunk; tok < end; tok += kCkTile, ++n) {
+          const int s = n % kCkStages;
+          int blk = block_tables[static_cast<size_t>(it.b) * table_width + tok / block_size];
+          if (blk < 0 || blk >= num_blocks) {
+            set_status(status, kStatusBadIndex);
+            blk = 0;
+          }
+          const int row = (blk * nkv + it.kvh) * block_size + tok % block_size;
+          ok = mbar_wait(&empty_bar[s], ((n / kCkStages) & 1) ^ 1, status);
+          if (!ok) break;
+          uint8_t* stg = smem + s * 2 * kCkTileBytes;
+          mbar_expect_tx(&full_bar[s], 2 * kCkTileBytes);
+          tma_load_2d(stg, &tm_k, &full_bar[s], 0, row);
+          tma_load_2d(stg + kCkBox, &tm_k, &full_bar[s], 64, row);
+          tma_load_2d(stg + kCkTileBytes, &tm_v, &full_bar[s], 0, row);
+          tma_load_2d(stg + kCkTileBytes + kCkBox, &tm_v, &full_bar[s], 64, row);
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+    }
+    return;
+  }
+
+  // -------------------------------------------------------------------- consumers (warps 0..3): 16 tokens of every tile each
+  for (int b = blockIdx.x; b < B; b += gridDim.x)       // padding rows (length 0): defined output
+    if (context_lens[b] <= 0)
+      for (int i = threadIdx.x; i < nq * kD; i += 128) out[static_cast<size_t>(b) * nq * kD + i] = __float2bfloat16_rn(0.f);
+  const int row = lane >> 2, quad = lane & 3;           // fragment coordinates: head of the group, column pair
+  const int mat = lane >> 3, mrow = lane & 7;           // ldmatrix: this lane supplies row `mrow` of matrix `mat`
+  int n = 0;
+  bool ok = true;                                       // once a wait has run out none is made any more, but every barrier still is
+  for (int item = blockIdx.x; chunk_item(context_lens, B, nkv, unit, parts, cap, direct != 0, item, nullptr, it); item += gridDim.x) {
+    const int qh0 = it.kvh * G, begin = it.c * it.chunk, end = min(it.len, begin + it.chunk);
+    if (begin >= end) continue;                         // uniform for the consumers
+    // the newest token (position len - 1) is not in the cache yet: the warp that owns its row of its tile prepares it now
+    const int newest = it.len - 1, row_new = newest % kCkTile;
+    const bool owner = fuse.qkv != nullptr && newest >= begin && newest < end && warp == row_new / 16;
+    DecodeNewToken fresh = {};
+    uint32_t qa[8][2];                                  // rows 0..G-1 = the heads of the group, the others zero; 8 steps of 16 dims
+    if (fuse.qkv != nullptr) {
+      const float* cs = fuse.rope != nullptr ? fuse.rope + static_cast<size_t>(min(max(newest, 0), fuse.rope_rows - 1)) * kD : nullptr;
+      for (int g = warp; g < G; g += 4) {
+        float x[16];
+        decode_norm_rope_head(fuse.qkv + static_cast<size_t>(it.b) * fuse.ld_qkv + static_cast<size_t>(qh0 + g) * kD, fuse.q_w, fuse.eps, cs, lane, x);
+        if (lane < 8) {
+          *reinterpret_cast<uint4*>(s_q + g * kD + 8 * lane) =
+              make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+          *reinterpret_cast<uint4*>(s_q + g * kD + 64 + 8 * lane) =
+              make_uint4(pack_bf16x2(x[8], x[9]), pack_bf16x2(x[10], x[11]), pack_bf16x2(x[12], x[13]), pack_bf16x2(x[14], x[15]));
+        }
+      }
+      if (owner) fresh = decode_new_token(fuse, it.b, it.kvh, nq, nkv, it.len, lane);
+      named_barrier_sync(1, 128);
+    }
+    {
+      const __nv_bfloat16* qp = (fuse.qkv != nullptr ? s_q : q + (static_cast<size_t>(it.b) * nq + qh0) * kD) + row * kD + 2 * quad;
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        qa[kk][0] = row < G ? *reinterpret_cast<const uint32_t*>(qp + kk * 16) : 0u;
+        qa[kk][1] = row < G ? *reinterpret_cast<const uint32_t*>(qp + kk * 16 + 8) : 0u;
+      }
+    }
+    float m_run = -INFINITY, l_run = 0.f;               // of head `row`; l is this lane's share until the end
+    float o[16][4];                                     // [..][0, 1]: sums of hi V, [2, 3]: of lo V, of the same head and dims
+#pragma unroll
+    for (int nb = 0; nb < 16; ++nb) o[nb][0] = o[nb][1] = o[nb][2] = o[nb][3] = 0.f;
+    for (int tok0 = begin; tok0 < end; tok0 += kCkTile, ++n) {
+      const int s = n % kCkStages;
+      ok = ok && mbar_wait(&full_bar[s], (n / kCkStages) & 1, status);
+      uint8_t* stg = smem + s * 2 * kCkTileBytes;
+      const uint32_t Ks = smem_u32(stg), Vs = Ks + kCkTileBytes;
+      if (owner && newest - tok0 < kCkTile) {           // its tile: the row is put in place, and into the cache for later steps
+        int blk = block_tables[static_cast<size_t>(it.b) * table_width + newest / block_size];
+        const bool to_cache = blk >= 0 && blk < num_blocks;
+        if (!to_cache) blk = 0;
+        const size_t off = ((static_cast<size_t>(blk) * nkv + it.kvh) * block_size + newest % block_size) * kD;
+        if (lane < 8) {
+          *reinterpret_cast<uint4*>(stg + (ck_addr(Ks, row_new, lane) - Ks)) = fresh.k_lo;
+          *reinterpret_cast<uint4*>(stg + (ck_addr(Ks, row_new, 8 + lane) - Ks)) = fresh.k_hi;
+          if (to_cache) {
+            *reinterpret_cast<uint4*>(k_cache + off + 8 * lane) = fresh.k_lo;
+            *reinterpret_cast<uint4*>(k_cache + off + 64 + 8 * lane) = fresh.k_hi;
+          }
+        }
+        *reinterpret_cast<uint2*>(stg + (ck_addr(Vs, row_new, lane >> 1) - Ks) + (lane & 1) * 8) = fresh.v;
+        if (to_cache) *reinterpret_cast<uint2*>(v_cache + off + lane * 4) = fresh.v;
+        fence_proxy_async_smem();                       // a later copy into this stage comes after these writes
+        __syncwarp();
+      }
+      const int r0 = warp * 16;
+      float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        uint32_t kb[4];
+        ldsm_x4(ck_addr(Ks, r0 + (mat >> 1) * 8 + mrow, 2 * kk + (mat & 1)), kb);
+        const uint32_t a[4] = {qa[kk][0], 0u, qa[kk][1], 0u};
+        mma16816(sc[0], a, kb[0], kb[1]);
+        mma16816(sc[1], a, kb[2], kb[3]);
+      }
+      // this lane: head `row`, tokens r0 + j * 8 + 2 * quad + {0, 1} of the tile
+      const int valid = end - tok0;
+      float mt = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          sc[j][e] = r0 + j * 8 + 2 * quad + e < valid ? sc[j][e] * scale_log2 : -INFINITY;
+          mt = fmaxf(mt, sc[j][e]);
+        }
+      mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 1));
+      mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 2));
+      const float m_new = fmaxf(m_run, mt);
+      const float m_use = m_new == -INFINITY ? 0.f : m_new;
+      const float alpha = exp2f(m_run - m_use);
+      float p[2][2], hi[2][2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          p[j][e] = exp2f(sc[j][e] - m_use);
+          hi[j][e] = decode_bf16_round(p[j][e]);
+        }
+      l_run = l_run * alpha + (p[0][0] + p[0][1] + p[1][0] + p[1][1]);
+      m_run = m_new;
+#pragma unroll
+      for (int nb = 0; nb < 16; ++nb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[nb][e] *= alpha;
+      const uint32_t pa[4] = {pack_bf16x2(hi[0][0], hi[0][1]), pack_bf16x2(p[0][0] - hi[0][0], p[0][1] - hi[0][1]),
+                              pack_bf16x2(hi[1][0], hi[1][1]), pack_bf16x2(p[1][0] - hi[1][0], p[1][1] - hi[1][1])};
+#pragma unroll
+      for (int dd = 0; dd < 8; ++dd) {
+        uint32_t vb[4];
+        ldsm_x4_trans(ck_addr(Vs, r0 + (mat & 1) * 8 + mrow, 2 * dd + (mat >> 1)), vb);
+        mma16816(o[2 * dd], pa, vb[0], vb[1]);
+        mma16816(o[2 * dd + 1], pa, vb[2], vb[3]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty_bar[s]);
+    }
+    // ---- publish the warp's state in the layout decode_merged reads, merge, store
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+    if (row < G) {
+      float* dst = s_acc + (warp * G + row) * kD + 2 * quad;
+#pragma unroll
+      for (int nb = 0; nb < 16; ++nb) *reinterpret_cast<float2*>(dst + nb * 8) = make_float2(o[nb][0] + o[nb][2], o[nb][1] + o[nb][3]);
+      if (quad == 0) {
+        s_acc[4 * G * kD + warp * G + row] = m_run;
+        s_acc[4 * G * kD + 4 * G + warp * G + row] = l_run;
+      }
+    }
+    named_barrier_sync(1, 128);
+    const int d = threadIdx.x;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      float M, L;
+      const float ov = decode_merged<G>(s_acc, g, d, M, L);
+      if (it.len <= it.chunk) {
+        out[(static_cast<size_t>(it.b) * nq + qh0 + g) * kD + d] = __float2bfloat16_rn(ov);
+      } else {
+        const size_t p = (static_cast<size_t>(it.b) * nq + qh0 + g) * max_chunks + it.c;
+        part_o[p * kD + d] = ov;
+        if (d == 0) *reinterpret_cast<float2*>(part_ml + p * 2) = make_float2(M, L);
+      }
+    }
+    named_barrier_sync(1, 128);                         // s_acc and s_q are the next item's
+  }
+}
+
+extern "C" int forge_make_tmap_2d(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, int elem_bytes);
+
+template <int G>
+static int launch_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
+                         int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk, int max_chunks, int parts, float scale_log2, unsigned* status,
+                         cudaStream_t stream, const DecodeFuse& fuse) {
+  constexpr int smem = kCkStages * 2 * kCkTileBytes + decode_merge_floats(G) * 4 + G * kD * 2 + 2 * kCkStages * 8 + 1024;
+  static_assert(ck_ctas_per_sm(G) * (smem + 1024) <= 228 * 1024, "CTAs per SM");
+  auto kern = decode_attn_chunk_kernel<G>;
+  FORGE_ENSURE_DYN_SMEM(kern, smem);
+  CUtensorMap tm_k, tm_v;
+  const uint64_t rows = static_cast<uint64_t>(num_blocks) * nkv * block_size;
+  if (forge_make_tmap_2d(&tm_k, kc, rows, kD, kD, kCkTile, 2) != 0 || forge_make_tmap_2d(&tm_v, vc, rows, kD, kD, kCkTile, 2) != 0) return -2;
+  // up to two waves of CTAs: one per item, dead ones included (they end at once, and no list is walked); else the live ones over one wave
+  const long long most = static_cast<long long>(B) * nkv * parts;
+  const int wave = ck_ctas_per_sm(G) * device_sm_count();
+  const int direct = most <= 2 * wave;
+  const dim3 grid(static_cast<unsigned>(direct ? most : wave));
+  return launch_kernel(kern, grid, dim3(kDecThreads), smem, stream, 0, tm_k, tm_v, static_cast<const __nv_bfloat16*>(q),
+                       static_cast<__nv_bfloat16*>(const_cast<void*>(kc)), static_cast<__nv_bfloat16*>(const_cast<void*>(vc)), bt, lens,
+                       static_cast<__nv_bfloat16*>(out), part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, chunk, max_chunks, parts,
+                       direct, scale_log2, status, fuse) == cudaSuccess ? 0 : -5;
+}
+
+// The attention kernel alone (partials of sequences of several chunks are merged by the caller); group = nq / nkv, 4..8.
+int launch_decode_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
+                         int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk, int max_chunks, int parts, float scale_log2, unsigned* status,
+                         cudaStream_t stream, const DecodeFuse& fuse) {
+#define FORGE_CK(G)                                                                                                                          \
+  case G:                                                                                                                                    \
+    return launch_chunks<G>(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, chunk, max_chunks, \
+                            parts, scale_log2, status, stream, fuse)
+  switch (nq / nkv) {
+    FORGE_CK(4);
+    FORGE_CK(5);
+    FORGE_CK(6);
+    FORGE_CK(7);
+    FORGE_CK(8);
+    default: return -1;
+  }
+#undef FORGE_CK
+}
+
+}  // namespace forge

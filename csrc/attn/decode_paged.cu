@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kDecThreads, decode_ctas_per_sm(G)) decode_att
     const __nv_bfloat16* __restrict__ q, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
     const int* __restrict__ block_tables, const int* __restrict__ context_lens, __nv_bfloat16* __restrict__ out,
     float* __restrict__ part_o, float* __restrict__ part_ml, int nq, int nkv, int block_size, int table_width, int num_blocks,
-    int chunk, int max_chunks, float scale_log2, unsigned* status, const DecodeFuse fuse) {
+    int unit, int max_chunks, int parts, float scale_log2, unsigned* status, const DecodeFuse fuse) {
   constexpr int kTileBytes = TILE * kD * 2;
   static_assert(TILE >= 16 && TILE <= 64 && (TILE & (TILE - 1)) == 0, "tile");
 
@@ -56,7 +56,8 @@ __global__ void __launch_bounds__(kDecThreads, decode_ctas_per_sm(G)) decode_att
   const int qh0 = kvh * (nq / nkv) + (blockIdx.x % groups_per_kv) * G;
   const int b = blockIdx.y;
   const int c = blockIdx.z;
-  const int len = decode_checked_len(context_lens, b, min(table_width * block_size, max_chunks * chunk), status);
+  const int len = decode_checked_len(context_lens, b, min(table_width * block_size, max_chunks * unit), status);
+  const int chunk = decode_chunk_tokens(len, unit, parts);
   const int tok_begin = c * chunk;
   if (tok_begin >= len) {                                // uniform for the CTA
     if (c == 0 && threadIdx.x < kD)                      // padding row (length 0): defined output
@@ -155,32 +156,86 @@ __global__ void __launch_bounds__(kDecThreads, decode_ctas_per_sm(G)) decode_att
   }
 }
 
-// Merge the per-chunk partials of sequences that span more than one chunk.
+// Merge the per-chunk partials of sequences that span more than one chunk.  The (max, sum) pairs are read by all threads at once and the
+// partial rows eight at a time: with one after another the merge of 47 chunks took 8.7 us, longer than it took to make half of them.
 __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                             const int* __restrict__ context_lens, __nv_bfloat16* __restrict__ out,
-                                                            int nq, int chunk, int max_chunks, int cap) {
+                                                            int nq, int unit, int max_chunks, int parts, int cap) {
+  __shared__ float s_w[kD], s_max[kD / 32];
   pdl_launch_dependents();
   pdl_wait();
   const int b = blockIdx.y, qh = blockIdx.x, d = threadIdx.x;
   const int len = decode_checked_len(context_lens, b, cap, nullptr);      // same clamp as the attention kernel, which reports it
+  const int chunk = decode_chunk_tokens(len, unit, parts);
   const int n = (len + chunk - 1) / chunk;
   if (n <= 1) return;
   const size_t base = (static_cast<size_t>(b) * nq + qh) * max_chunks;
-  float M = -INFINITY;
-  for (int c = 0; c < n; ++c) M = fmaxf(M, part_ml[(base + c) * 2]);
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + base;
+  if (n <= 8) {                                          // everything at once, nothing between threads
+    float2 x[8];
+    float v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      x[c] = c < n ? ml[c] : make_float2(-INFINITY, 0.f);
+      v[c] = c < n ? part_o[(base + c) * kD + d] : 0.f;
+    }
+    float M = x[0].x, L = 0.f, O = 0.f;
+#pragma unroll
+    for (int c = 1; c < 8; ++c) M = fmaxf(M, x[c].x);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float w = c < n ? x[c].y * exp2f(x[c].x - M) : 0.f;
+      L += w;
+      O += v[c] * w;
+    }
+    out[(static_cast<size_t>(b) * nq + qh) * kD + d] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+    return;
+  }
+  const float2 first = d < n ? ml[d] : make_float2(-INFINITY, 0.f);
+  float M = first.x;
+  for (int c = d + kD; c < n; c += kD) M = fmaxf(M, ml[c].x);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  if ((d & 31) == 0) s_max[d >> 5] = M;
+  __syncthreads();
+  M = fmaxf(fmaxf(s_max[0], s_max[1]), fmaxf(s_max[2], s_max[3]));
   float L = 0.f, O = 0.f;
-  for (int c = 0; c < n; ++c) {
-    const float w = part_ml[(base + c) * 2 + 1] * exp2f(part_ml[(base + c) * 2] - M);
-    L += w;
-    O += part_o[(base + c) * kD + d] * w;
+  for (int c0 = 0; c0 < n; c0 += kD) {
+    const float2 x = c0 == 0 ? first : c0 + d < n ? ml[c0 + d] : make_float2(-INFINITY, 0.f);
+    if (c0 > 0) __syncthreads();
+    s_w[d] = x.y * exp2f(x.x - M);
+    __syncthreads();
+    const int m = min(kD, n - c0);
+    const float* src = part_o + (base + c0) * kD + d;
+    int c = 0;
+    for (; c + 8 <= m; c += 8) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = src[static_cast<size_t>(c + i) * kD];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        L += s_w[c + i];
+        O += v[i] * s_w[c + i];
+      }
+    }
+    for (; c < m; ++c) {
+      L += s_w[c];
+      O += src[static_cast<size_t>(c) * kD] * s_w[c];
+    }
   }
   out[(static_cast<size_t>(b) * nq + qh) * kD + d] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+}
+
+static int launch_decode_combine(const float* part_o, const float* part_ml, const int* lens, void* out, int B, int nq, int chunk, int max_chunks, int parts, int cap,
+                                 cudaStream_t stream) {
+  return launch_kernel(decode_combine_kernel, dim3(nq, B), dim3(kD), 0, stream, 0, part_o, part_ml, lens, static_cast<__nv_bfloat16*>(out), nq, chunk,
+                       max_chunks, parts, cap) == cudaSuccess ? 0 : -5;
 }
 
 template <int G, int TILE>
 static int launch_decode(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o,
                          float* part_ml, int B, int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk,
-                         int max_chunks, float scale_log2, unsigned* status, cudaStream_t stream, const DecodeFuse& fuse) {
+                         int max_chunks, int parts, float scale_log2, unsigned* status, cudaStream_t stream, const DecodeFuse& fuse) {
   constexpr int kTileBytes = TILE * kD * 2;
   constexpr int merge_bytes = decode_merge_floats(G) * 4;
   constexpr int ring = kDecStages * 2 * kTileBytes;
@@ -188,21 +243,20 @@ static int launch_decode(const void* q, const void* kc, const void* vc, const in
   auto kern = decode_attn_kernel<G, TILE>;
   FORGE_ENSURE_DYN_SMEM(kern, smem);
   const int groups_per_kv = (nq / nkv) / G;
-  dim3 grid(nkv * groups_per_kv, B, max_chunks);
+  dim3 grid(nkv * groups_per_kv, B, parts);
   if (launch_kernel(kern, grid, dim3(kDecThreads), smem, stream, 0, static_cast<const __nv_bfloat16*>(q),
                     static_cast<__nv_bfloat16*>(const_cast<void*>(kc)), static_cast<__nv_bfloat16*>(const_cast<void*>(vc)), bt, lens,
                     static_cast<__nv_bfloat16*>(out), part_o, part_ml, nq, nkv, block_size, table_width, num_blocks, chunk,
-                    max_chunks, scale_log2, status, fuse) != cudaSuccess)
+                    max_chunks, parts, scale_log2, status, fuse) != cudaSuccess)
     return -5;
-  if (max_chunks > 1) {
-    dim3 g2(nq, B);
-    if (launch_kernel(decode_combine_kernel, g2, dim3(kD), 0, stream, 0, static_cast<const float*>(part_o),
-                      static_cast<const float*>(part_ml), lens, static_cast<__nv_bfloat16*>(out), nq, chunk, max_chunks,
-                      std::min(table_width * block_size, max_chunks * chunk)) != cudaSuccess)
-      return -5;
-  }
+  if (max_chunks > 1)
+    return launch_decode_combine(part_o, part_ml, lens, out, B, nq, chunk, max_chunks, parts, std::min(table_width * block_size, max_chunks * chunk), stream);
   return 0;
 }
+
+int launch_decode_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
+                         int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk, int max_chunks, int parts, float scale_log2, unsigned* status,
+                         cudaStream_t stream, const DecodeFuse& fuse);
 
 // q [B, nq, 128] bf16; caches [num_blocks, nkv, block_size, 128] bf16; block_tables [B, table_width]; out [B, nq * 128].
 // part_o: fp32 [B, nq, max_chunks, 128], part_ml: fp32 [B, nq, max_chunks, 2] (may be null when max_chunks == 1).
@@ -219,9 +273,20 @@ static int decode_chunked_impl(const void* q, const void* kc, const void* vc, co
   const int group = nq / nkv;
   const int G = decode_group_slice(group);
   const float sl2 = scale * 1.4426950408889634f;
+  // Very few sequences: at most 24 chunks each, more of them cost the merge more than they save (3001 tokens of 32 / 8 heads: 47 chunks 15.5 us, 24: 13.3).
+  const int parts = B * nkv < 32 ? std::min(max_chunks, 24) : max_chunks;
+  // Groups of 4 to 8 heads, cache blocks of 64 tokens and more: on the tensor cores (decode_chunks.cu); TMA wants 16-byte rows.  With two heads per
+  // KV head the CUDA cores keep up with the stream and their kernel starts faster (2 sequences 12.0 us against 13.8, 40: 44 against 53); with four
+  // they do not (13 sequences: 31.7 against 22.4).
+  if (tile == 64 && group >= 4 && group <= 8 && ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0) {
+    const int rc = launch_decode_chunks(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, chunk, max_chunks, parts, sl2,
+                                        status, stream, fuse);
+    if (rc != 0 || max_chunks <= 1) return rc;
+    return launch_decode_combine(part_o, part_ml, lens, out, B, nq, chunk, max_chunks, parts, std::min(table_width * block_size, max_chunks * chunk), stream);
+  }
 #define FORGE_DEC(GG, TT)                                                                                                   \
   return launch_decode<GG, TT>(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, \
-                               chunk, max_chunks, sl2, status, stream, fuse)
+                               chunk, max_chunks, parts, sl2, status, stream, fuse)
   if (tile == 64) {
     if (G == 5) FORGE_DEC(5, 64);
     if (G == 4) FORGE_DEC(4, 64);

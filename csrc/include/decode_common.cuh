@@ -277,6 +277,12 @@ __device__ __forceinline__ float decode_merged(const float* s_acc, int g, int d,
   return L > 0.f ? O / L : 0.f;
 }
 
+// Tokens of a context chunk of a sequence: the smallest multiple of `unit` with which it has at most `parts` chunks.
+__device__ __forceinline__ int decode_chunk_tokens(int len, int unit, int parts) {
+  const int units = (len + unit - 1) / unit;
+  return units <= parts ? unit : unit * ((units + parts - 1) / parts);
+}
+
 constexpr int decode_merge_floats(int G) { return 4 * G * kD + 8 * G; }
 
 }  // namespace forge

@@ -580,6 +580,29 @@ def test_decode_attention_cuda_core_variant_for_groups_of_4_and_5(ops, k_lens, n
     ops.check_status()
 
 
+@pytest.mark.parametrize("k_lens,nq,nkv,bs,chunk,max_chunks", [
+    ([1, 63, 64, 65, 0, 128, 129, 700], 32, 8, 256, 64, 16),           # edges of tiles and chunks, a padding row, every sequence cut
+    ([2000, 5], 8, 2, 64, 64, 32),                                     # at most 24 chunks: longer ones than asked for
+    ([0, 640, 641, 1], 10, 2, 128, 128, 6), ([300, 511], 12, 2, 256, 64, 8), ([300, 511], 7, 1, 256, 256, 2), ([900] * 3, 16, 2, 512, 1024, 1),
+    ([17 * i % 900 for i in range(70)], 32, 8, 256, 64, 15),           # more items than two waves: walked as a list, three ballots of sequences
+])
+def test_decode_attention_chunks_on_tensor_cores(ops, k_lens, nq, nkv, bs, chunk, max_chunks):
+    """Groups of 4 to 8 heads; the weights keep 16 bits, so what is left is the rounding of the bf16 result (2^-9 of values of unit size)."""
+    q, kc, vc, b = _paged_case([1] * len(k_lens), k_lens, nq, nkv, bs, seed=4)
+    want = ref.attention(q, kc, vc, b.cu_seqlens_q, b.context_lens, b.block_tables, 128 ** -0.5, b.num_seqs)
+    B = len(k_lens)
+    part_o = torch.full((B * nq * max_chunks * 128,), float("nan"), device="cuda")
+    part_ml = torch.full((B * nq * max_chunks * 2,), float("nan"), device="cuda")
+    got = torch.full((B, nq * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.C.decode_attention(q, kc, vc, b.block_tables, b.context_lens, got, part_o, part_ml, chunk, max_chunks, 128 ** -0.5, ops.status)
+    for i, n in enumerate(k_lens):
+        if n == 0:
+            assert torch.count_nonzero(got[i]) == 0
+        else:
+            _close(got[i], want.view(B, -1)[i], 2e-2, 2e-2)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("batch,lo,hi,nq,nkv", [(64, 100, 1500, 16, 8), (200, 1, 700, 16, 8), (300, 3000, 3100, 8, 2), (7, 1, 4000, 32, 8),
                                                 (70, 100, 2500, 64, 8)])
 def test_decode_attention_flat_partition_many_sequences(ops, batch, lo, hi, nq, nkv, monkeypatch):
