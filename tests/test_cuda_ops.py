@@ -659,6 +659,25 @@ def test_prefill_attention_two_tiles_per_cta(ops, q_lens, k_lens, nq, nkv, bs):
     ops.check_status()
 
 
+def test_prefill_attention_does_not_depend_on_the_batch(ops):
+    """A sequence alone (one query tile per CTA) and the same one among others (two): the same bits, so a prompt computed in portions or beside
+    others gives the tokens it gives by itself."""
+    lens = [1000, 333, 129, 64] + [300] * 8
+    q, kc, vc, b = _paged_case(lens, lens, 16, 8, 256, seed=5)
+    b.is_prefill = True
+    whole = ops.attention(q, kc, vc, b, 128 ** -0.5)
+    at = 0
+    for i, n in enumerate(lens[:4]):
+        one = _Batch()
+        one.is_prefill, one.num_seqs, one.padded_seqs, one.table_width = True, 1, 1, b.table_width
+        one.cu_seqlens_q = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+        one.context_lens, one.block_tables = b.context_lens[i:i + 1].contiguous(), b.block_tables[i:i + 1].contiguous()
+        one.max_seqlen_q = one.max_seqlen_k = n
+        assert torch.equal(ops.attention(q[at:at + n].contiguous(), kc, vc, one, 128 ** -0.5), whole[at:at + n])
+        at += n
+    ops.check_status()
+
+
 # ----------------------------------------------------------------------------- sampler
 def _header(step, seed):
     h = torch.zeros(16, dtype=torch.int32)
