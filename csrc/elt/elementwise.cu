@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(128) qk_norm_rope_store128_kernel(
       }
       float ss = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss += a[e] * a[e] + b[e] * b[e];
+      for (int e = 0; e < 8; ++e) ss = add_squares(a[e], b[e], ss);
       const unsigned gmask = 0xFFu << (sub * 8);        // the four 8-lane groups may hold different kinds of heads
       ss += __shfl_xor_sync(gmask, ss, 1);
       ss += __shfl_xor_sync(gmask, ss, 2);
@@ -311,11 +311,7 @@ __global__ void __launch_bounds__(128) qk_norm_rope_store128_kernel(
       }
       if (do_rope) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float x1 = a[e], x2 = b[e];
-          a[e] = x1 * cosv[e] - x2 * sinv[e];
-          b[e] = x2 * cosv[e] + x1 * sinv[e];
-        }
+        for (int e = 0; e < 8; ++e) rotate_pair(a[e], b[e], cosv[e], sinv[e]);
       }
       lo = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]), pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
       hi = make_uint4(pack_bf16x2(b[0], b[1]), pack_bf16x2(b[2], b[3]), pack_bf16x2(b[4], b[5]), pack_bf16x2(b[6], b[7]));

@@ -711,6 +711,137 @@ gemm_tokens_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
   }
 }
 
+// What the kEpiQkv epilogue needs of a token row, and its first cos / sin values: fetched while the tile is still being multiplied.
+struct QkvRow {
+  float row_scale;
+  bool live, slot_ok;
+  size_t first;               // the row of KV head 0 in the cache
+  const float* cs;
+  float cw[16], sw[16];
+};
+
+__device__ __forceinline__ void qkv_turn_factors(const float* cs, int c, float (&cw)[16], float (&sw)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 4) {
+    const float4 cv = *reinterpret_cast<const float4*>(cs + c + i), sv = *reinterpret_cast<const float4*>(cs + 64 + c + i);
+    cw[i] = cv.x; cw[i + 1] = cv.y; cw[i + 2] = cv.z; cw[i + 3] = cv.w;
+    sw[i] = sv.x; sw[i + 1] = sv.y; sw[i + 2] = sv.z; sw[i + 3] = sv.w;
+  }
+}
+
+__device__ __forceinline__ void qkv_fetch_row(QkvRow& q, int h0, int r, int m_total, const GemmFuse& fuse, const GemmQkv& qk, unsigned* status) {
+  q.live = r < m_total;
+  const int slot = q.live ? qk.slots[r] : -1;
+  int pos = q.live && qk.do_rope ? qk.positions[r] : 0;
+  q.row_scale = fuse_row_scale(fuse, r, m_total);
+  pos = pos < 0 ? 0 : (pos >= qk.rope_rows ? qk.rope_rows - 1 : pos);
+  q.cs = qk.rope + static_cast<size_t>(pos) * 128;
+  if (qk.do_rope && h0 < qk.nq + qk.nkv) qkv_turn_factors(q.cs, 0, q.cw, q.sw);
+  q.slot_ok = slot >= 0 && slot < qk.num_slots;
+  if (slot >= qk.num_slots) set_status(status, kStatusBadIndex);
+  const unsigned blk = q.slot_ok ? static_cast<unsigned>(slot) / static_cast<unsigned>(qk.block_size) : 0u;
+  q.first = static_cast<size_t>(blk) * qk.nkv * qk.block_size + (q.slot_ok ? slot - blk * qk.block_size : 0u);
+}
+
+// The kEpiQkv epilogue of a 256-column tile: one token row of two heads h0, h0 + 1 per thread, which share its cos / sin values (the
+// projection streams its operands at the rate of the SM's L2 port, so the table is read once per row, not once per head).
+__device__ __forceinline__ void qkv_pair_epilogue(uint32_t tacc, int h0, int r, QkvRow& q, const GemmQkv& qk) {
+  const int heads = qk.nq + 2 * qk.nkv;
+  const bool live = q.live, slot_ok = q.slot_ok;
+  const float row_scale = q.row_scale;
+  const size_t first = q.first;
+  float (&cw)[16] = q.cw;
+  float (&sw)[16] = q.sw;
+  __nv_bfloat16* dst[2];
+  const __nv_bfloat16* nw[2];
+  float inv[2];
+  bool turn[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int h = h0 + k;
+    const bool is_q = h < qk.nq, is_k = !is_q && h < qk.nq + qk.nkv;
+    dst[k] = nullptr;
+    if (live && h < heads) {
+      if (is_q) dst[k] = qk.q_out + (static_cast<size_t>(r) * qk.nq + h) * 128;
+      else if (slot_ok)
+        dst[k] = (is_k ? qk.k_cache : qk.v_cache) + (first + static_cast<size_t>(is_k ? h - qk.nq : h - qk.nq - qk.nkv) * qk.block_size) * 128;
+    }
+    nw[k] = is_q ? qk.qw : is_k ? qk.kw : nullptr;
+    turn[k] = (is_q || is_k) && qk.do_rope != 0;
+    inv[k] = 1.f;
+    if (nw[k] != nullptr) {                                             // uniform over the tile
+      float ss = 0.f;                                                   // in the order of qk_norm_rope_store128_kernel
+#pragma unroll 1
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t va[32], vb[32];
+        tmem_ld_x32(tacc + k * 128 + c, va);
+        tmem_ld_x32(tacc + k * 128 + 64 + c, vb);
+        tmem_ld_wait();
+        float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          part[j >> 3] = add_squares(bf16_round_g(__uint_as_float(va[j]) * row_scale), bf16_round_g(__uint_as_float(vb[j]) * row_scale), part[j >> 3]);
+        ss += (part[0] + part[1]) + (part[2] + part[3]);
+      }
+      inv[k] = rsqrtf(ss / 128.f + qk.eps);
+    }
+  }
+#pragma unroll 1
+  for (int c = 0; c < 64; c += 16) {                                    // columns [c, c + 16) and their partners 64 further
+    float cw_next[16], sw_next[16];
+    const bool fetch = turn[0] && c + 16 < 64;                          // (a tile whose first head does not turn has no head that does)
+    if (fetch) qkv_turn_factors(q.cs, c + 16, cw_next, sw_next);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      uint32_t va[16], vb[16];
+      tmem_ld_x16(tacc + k * 128 + c, va);
+      tmem_ld_x16(tacc + k * 128 + 64 + c, vb);
+      tmem_ld_wait();
+      float a[16], b[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        a[j] = bf16_round_g(__uint_as_float(va[j]) * row_scale);
+        b[j] = bf16_round_g(__uint_as_float(vb[j]) * row_scale);
+      }
+      if (nw[k] != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 8) {
+          const uint4 wa = *reinterpret_cast<const uint4*>(nw[k] + c + i), wb = *reinterpret_cast<const uint4*>(nw[k] + 64 + c + i);
+          const uint32_t ra[4] = {wa.x, wa.y, wa.z, wa.w}, rb[4] = {wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int j = i + 2 * e;
+            a[j] = bf16_round_g(bf16_round_g(a[j] * inv[k]) * bf16_lo(ra[e]));
+            a[j + 1] = bf16_round_g(bf16_round_g(a[j + 1] * inv[k]) * bf16_hi(ra[e]));
+            b[j] = bf16_round_g(bf16_round_g(b[j] * inv[k]) * bf16_lo(rb[e]));
+            b[j + 1] = bf16_round_g(bf16_round_g(b[j + 1] * inv[k]) * bf16_hi(rb[e]));
+          }
+        }
+      }
+      if (turn[k]) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) rotate_pair(a[j], b[j], cw[j], sw[j]);
+      }
+      if (dst[k] != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 16; j += 8) {
+          *reinterpret_cast<uint4*>(dst[k] + c + j) =
+              make_uint4(pack_bf16x2(a[j], a[j + 1]), pack_bf16x2(a[j + 2], a[j + 3]), pack_bf16x2(a[j + 4], a[j + 5]), pack_bf16x2(a[j + 6], a[j + 7]));
+          *reinterpret_cast<uint4*>(dst[k] + 64 + c + j) =
+              make_uint4(pack_bf16x2(b[j], b[j + 1]), pack_bf16x2(b[j + 2], b[j + 3]), pack_bf16x2(b[j + 4], b[j + 5]), pack_bf16x2(b[j + 6], b[j + 7]));
+        }
+      }
+    }
+    if (fetch) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        cw[i] = cw_next[i];
+        sw[i] = sw_next[i];
+      }
+    }
+  }
+}
+
 // =========================================================================================================
 // many tokens, CTA pairs: one UMMA of M = 256 tokens x N = 256 features per pair of SMs (cta_group::2)
 // =========================================================================================================
@@ -740,7 +871,7 @@ template <int kEpi>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                  __nv_bfloat16* __restrict__ out, int ldo, int m_total, int n_total, int K, int dual_off, unsigned* status,
-                 const TpPush push, const GemmFuse fuse, const GemmStreamK sk) {
+                 const TpPush push, const GemmFuse fuse, const GemmStreamK sk, const GemmQkv qk) {
   using Cfg = PairCfg<kEpi>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -860,25 +991,31 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
       tile_coords(t, m_tiles, n_tiles, kRasterGroupPair, mt, nt);
       const int r = mt * 2 * kBlockR + rank * kBlockR + quad * 32 + lane;
       const int c0 = nt * Cfg::kBlockN;
+      [[maybe_unused]] QkvRow qrow;
+      if constexpr (kEpi == kEpiQkv) qkv_fetch_row(qrow, c0 / 128, r, m_total, fuse, qk, status);
       const bool ok = mbar_wait(&acc_full[buf], (n >> 1) & 1, status);
       tcgen05_fence_after();
       const bool whole = kb0 == 0 && kb1 == num_kb;
       const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * Cfg::kAccCols;
       const uint32_t leader_empty = dsmem_addr(smem_u32(&acc_empty[buf]), 0);
       bool released = false;
-      SkTile tile = {};
-      if (ok && !whole) {
-        const long long u_seg = static_cast<long long>(t) * sched.num_kg + kb0 / sched.kgroup;
-        sk_dump<Cfg::kAccCols>(tacc, sk.ws + (static_cast<size_t>(blockIdx.x) * 2 + (u_seg == sched.u_begin ? 0 : 1)) * kSkSlotFloats,
-                               quad * 32 + lane, r < m_total);
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(leader_empty);
-        released = true;
-        if (!sk.defer) tile = sk_arrive(sk, t * 2 + rank, sk_flag, warp == 2 && lane == 0, t, num_tiles, sched.num_kg, pairs, 2, rank);
+      if constexpr (kEpi == kEpiQkv) {                   // never with parts of K
+        if (ok) qkv_pair_epilogue(tacc, c0 / 128, r, qrow, qk);
+      } else {
+        SkTile tile = {};
+        if (ok && !whole) {
+          const long long u_seg = static_cast<long long>(t) * sched.num_kg + kb0 / sched.kgroup;
+          sk_dump<Cfg::kAccCols>(tacc, sk.ws + (static_cast<size_t>(blockIdx.x) * 2 + (u_seg == sched.u_begin ? 0 : 1)) * kSkSlotFloats,
+                                 quad * 32 + lane, r < m_total);
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(leader_empty);
+          released = true;
+          if (!sk.defer) tile = sk_arrive(sk, t * 2 + rank, sk_flag, warp == 2 && lane == 0, t, num_tiles, sched.num_kg, pairs, 2, rank);
+        }
+        if (ok && (whole || tile.n > 0))
+          tile_epilogue<Cfg::kBlockN, kEpi>(tacc, whole, tile, sk.ws, quad * 32 + lane, r, c0, m_total, n_total, out, ldo, fuse);
       }
-      if (ok && (whole || tile.n > 0))
-        tile_epilogue<Cfg::kBlockN, kEpi>(tacc, whole, tile, sk.ws, quad * 32 + lane, r, c0, m_total, n_total, out, ldo, fuse);
       if (!released) {
         tcgen05_fence_before();
         __syncwarp();
@@ -1501,7 +1638,7 @@ static int launch_tokens(const void* x, int ldx, const void* w, int w_rows, int 
 template <int kEpi>
 static int launch_pair(const void* x, int ldx, const void* w, int w_rows, int ldw, __nv_bfloat16* out, int ldo, int M, int n_out,
                        int K, unsigned* status, cudaStream_t stream, const TpPush& push, const GemmFuse& fuse, int kgroup,
-                       int w_dynamic = 0, int defer_splits = 0) {
+                       int w_dynamic = 0, int defer_splits = 0, const GemmQkv& qk = GemmQkv{}) {
   using Cfg = PairCfg<kEpi>;
   w_dynamic |= fuse.w_dynamic;
   CUtensorMap tm_x, tm_w;
@@ -1516,17 +1653,19 @@ static int launch_pair(const void* x, int ldx, const void* w, int w_rows, int ld
   int pairs = tiles < max_pairs ? tiles : max_pairs;
   GemmStreamK sk = {nullptr, nullptr, 0, w_dynamic, 0};
   const StreamKWorkspace* wsp = streamk_workspace();
-  if (defer_splits > 1 && wsp != nullptr && push.size <= 1) {
-    const int kg = (num_kb + defer_splits - 1) / defer_splits;
-    const int num_kg = (num_kb + kg - 1) / kg;
-    const long long units = static_cast<long long>(tiles) * num_kg;
-    if (num_kg > 1 && units <= max_pairs && 2 * units <= wsp->ctas) {
-      sk = GemmStreamK{wsp->ws, wsp->counters, kg, w_dynamic, 1};
-      if (launch_kernel_cluster_x(kern, dim3(static_cast<unsigned>(2 * units)), dim3(kGemmThreads), Cfg::kSmemBytes, stream, 2, tm_x, tm_w,
-                                  out, ldo, M, n_out, K, n_out, status, push, fuse, sk) != cudaSuccess)
-        return -5;
-      return launch_finish<kEpi>(sk, tiles, m_tiles, n_tiles, num_kg, static_cast<int>(units), 1, Cfg::kBlockN, kRasterGroupPair, out, ldo,
-                                 M, n_out, fuse, stream);
+  if constexpr (kEpi != kEpiQkv) {
+    if (defer_splits > 1 && wsp != nullptr && push.size <= 1) {
+      const int kg = (num_kb + defer_splits - 1) / defer_splits;
+      const int num_kg = (num_kb + kg - 1) / kg;
+      const long long units = static_cast<long long>(tiles) * num_kg;
+      if (num_kg > 1 && units <= max_pairs && 2 * units <= wsp->ctas) {
+        sk = GemmStreamK{wsp->ws, wsp->counters, kg, w_dynamic, 1};
+        if (launch_kernel_cluster_x(kern, dim3(static_cast<unsigned>(2 * units)), dim3(kGemmThreads), Cfg::kSmemBytes, stream, 2, tm_x, tm_w,
+                                    out, ldo, M, n_out, K, n_out, status, push, fuse, sk, qk) != cudaSuccess)
+          return -5;
+        return launch_finish<kEpi>(sk, tiles, m_tiles, n_tiles, num_kg, static_cast<int>(units), 1, Cfg::kBlockN, kRasterGroupPair, out, ldo,
+                                   M, n_out, fuse, stream);
+      }
     }
   }
   if (kgroup > 0) {
@@ -1539,7 +1678,7 @@ static int launch_pair(const void* x, int ldx, const void* w, int w_rows, int ld
     }
   }
   return launch_kernel_cluster_x(kern, dim3(2 * pairs), dim3(kGemmThreads), Cfg::kSmemBytes, stream, 2, tm_x, tm_w, out, ldo, M, n_out,
-                                 K, n_out, status, push, fuse, sk) == cudaSuccess ? 0 : -5;
+                                 K, n_out, status, push, fuse, sk, qk) == cudaSuccess ? 0 : -5;
 }
 
 // Cluster size (K splits) of the decode kernel.  Measured on B200 (sweeps over token tile x splits x ring depth for
@@ -1829,6 +1968,12 @@ extern "C" int forge_gemm_bf16_qkv(const void* x, int ldx, const void* w, int ld
                 nq, nkv, block_size, do_rope, num_slots};
   const int n_out = (nq + 2 * nkv) * 128;
   TpPush none = {};
+  // Prompts: the CTA-pair kernel, like the plain projection.  A tile's 64 KB of cos / sin values and the longer epilogue hide behind
+  // the products; what goes is a pass over q, k and v (written, read and written again).
+  // With the pass as a kernel of its own / in here: 3777 tokens, K 4096, 32 + 16 heads: 180 / 149 us; 2048: 111 / 99; 8192, K 2560: 224 / 206.
+  // With K 1024 the products of a tile are shorter than its epilogue (15717 tokens, 16 + 16 heads: 162 / 165; 2000: 32 / 36): callers
+  // keep the two kernels there.
+  if (M > 256) return launch_pair<kEpiQkv>(x, ldx, w, n_out, ldw, nullptr, 0, M, n_out, K, status, stream, none, fuse, 0, 0, 0, qk);
   return launch_tokens<128, kEpiQkv>(x, ldx, w, n_out, ldw, nullptr, 0, M, n_out, K, status, stream, none, fuse, GemmSample{}, 0, 0, 0, qk);
 }
 

@@ -376,6 +376,29 @@ def test_qkv_gemm_with_norm_rope_and_cache_store_in_its_epilogue(ops, T, K, nq, 
     ops.check_status()
 
 
+@pytest.mark.parametrize("T,K,nq,nkv,bs,folded", [(257, 1024, 16, 8, 256, True), (511, 512, 5, 1, 64, False), (1025, 4096, 32, 8, 256, True),
+                                                 (3000, 256, 3, 3, 16, True), (700, 1024, 2, 1, 128, False)])
+def test_qkv_gemm_of_prompts_with_norm_rope_and_cache_store_in_its_epilogue(ops, T, K, nq, nkv, bs, folded):
+    """More than 256 rows: CTA pairs, two heads per tile (q and k, k and v in one tile; an odd number of heads; ragged last rows)."""
+    test_qkv_gemm_with_norm_rope_and_cache_store_in_its_epilogue(ops, T, K, nq, nkv, bs, folded)
+
+
+@pytest.mark.parametrize("T,K,nq,nkv", [(300, 2048, 16, 8), (1500, 4096, 5, 1)])
+def test_qkv_gemm_of_prompts_gives_the_bits_of_the_two_kernels(ops, T, K, nq, nkv):
+    torch.manual_seed(T)
+    x, w = _rand(T, K), _rand((nq + 2 * nkv) * 128, K, scale=0.05)
+    qw, kw = _rand(128, scale=0.2) + 1, _rand(128, scale=0.2) + 1
+    ssq = (x.float() ** 2).view(T, K // 128, -1).sum(-1).contiguous()
+    table = ref.rope_table(4096, 128, 1e6, "cuda")
+    pos = torch.randint(0, 4096, (T,), dtype=torch.int32, device="cuda")
+    slots = torch.randperm(2048, device="cuda")[:T].to(torch.int32)
+    caches = [torch.zeros(8, nkv, 256, 128, dtype=BF, device="cuda") for _ in range(4)]
+    got = ops.linear_qkv_rope_store(x, w, ssq, 1e-6, qw, kw, 1e-6, table, pos, slots, caches[0], caches[1], nq, nkv)
+    want = ops.qk_norm_rope_store(ops.linear_scaled(x, w, ssq, 1e-6), qw, kw, 1e-6, table, pos, slots, caches[2], caches[3], nq, nkv, 128)
+    assert torch.equal(got.view(-1), want.view(-1)) and torch.equal(caches[0], caches[2]) and torch.equal(caches[1], caches[3])
+    ops.check_status()
+
+
 def test_embedding_sum_of_squares(ops):
     V, H, T = 512, 1024, 37
     table = _rand(V, H)

@@ -162,7 +162,7 @@ class Qwen3ForCausalLM:
         ops, layers = self.ops, self.layers
         residual, ssq_a, ssq_b = ops.embedding_ssq(batch.input_ids, self.embed_tokens.weight, self.embed_tokens.vocab_start)
         fused_decode = (not batch.is_prefill and self.head_dim == 128 and batch.padded_seqs <= ops.fused_qkv_max_batch)
-        in_gemm = not batch.is_prefill and ops.qkv_rope_store_in_gemm(residual.shape[0], self.head_dim, layers[0].qkv_proj.weight)
+        in_gemm = ops.qkv_rope_store_in_gemm(residual.shape[0], self.head_dim, layers[0].qkv_proj.weight, batch.is_prefill)
         for i, l in enumerate(layers):
             kc, vc = self.kv_cache[i, 0], self.kv_cache[i, 1]
             if in_gemm:         # norm, rotation and cache write in the projection's epilogue: one launch less per block
@@ -199,8 +199,8 @@ class Qwen3ForCausalLM:
         # layer; at large batches the attention kernel is bandwidth-bound and the extra work per sequence costs more)
         fused_decode = (not batch.is_prefill and self.head_dim == 128 and hasattr(ops, "decode_attention_qkv")
                         and batch.padded_seqs <= ops.fused_qkv_max_batch)
-        in_gemm = (not batch.is_prefill and hasattr(ops, "qkv_rope_store_in_gemm") and getattr(layers[0].qkv_proj, "bias", None) is None
-                   and ops.qkv_rope_store_in_gemm(x.shape[0], self.head_dim, layers[0].qkv_proj.weight))
+        in_gemm = (hasattr(ops, "qkv_rope_store_in_gemm") and getattr(layers[0].qkv_proj, "bias", None) is None
+                   and ops.qkv_rope_store_in_gemm(x.shape[0], self.head_dim, layers[0].qkv_proj.weight, batch.is_prefill))
         for i, l in enumerate(layers):
             kc, vc = self.kv_cache[i, 0], self.kv_cache[i, 1]
             if in_gemm:

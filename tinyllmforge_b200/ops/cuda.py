@@ -262,11 +262,16 @@ class CudaOps(MixerOps, HybridOps):
                                   num_heads, num_kv_heads, do_rope, self.status)
         return q
 
-    def qkv_rope_store_in_gemm(self, rows: int, head_dim: int, weight) -> bool:
-        """Decode steps of 33..256 rows with head_dim 128 and a bf16 qkv weight: the projection's epilogue does the per-head
-        norm, the rotation and the cache write (tiles of 128 features = one head)."""
-        return (self.qkv_epilogue and head_dim == 128 and self.qkv_epilogue_min_rows <= rows <= 256
-                and not isinstance(weight, Fp8BlockWeight) and weight.dtype == torch.bfloat16)
+    def qkv_rope_store_in_gemm(self, rows: int, head_dim: int, weight, prefill: bool = False) -> bool:
+        """Whether the epilogue of the qkv projection does the per-head norm, the rotation and the cache write: steps of more than 256
+        rows of a hidden size from 2048 (CTA-pair kernel, two heads per tile; measured 180 -> 149 us with 3777 tokens of size 4096,
+        224 -> 206 with 8192 of 2560, but 162 -> 165 with 15717 of 1024, whose products are too short to hide the epilogue), and, if asked
+        for, decode steps of 33..256 (tiles of 128 features = one head); with head_dim 128 and a bf16 qkv weight."""
+        if head_dim != 128 or isinstance(weight, Fp8BlockWeight) or weight.dtype != torch.bfloat16:
+            return False
+        if rows > 256:
+            return weight.shape[1] >= 2048
+        return self.qkv_epilogue and self.qkv_epilogue_min_rows <= rows and not prefill
 
     def linear_qkv_rope_store(self, x, w, ssq_row, in_eps, q_weight, k_weight, eps, table, positions, slot_mapping, k_cache, v_cache,
                               num_heads, num_kv_heads, do_rope=True):
