@@ -399,13 +399,14 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
-// The rotation of a pair, and a step of the sum of squares of a head's halves, rounded alike wherever they are computed.
+// The rotation of a pair, and a step of the sum of squares of a head's halves, rounded alike wherever they are computed: in the order in
+// which qk_norm_rope_store128_kernel has always rounded them, so that a head's bits stay what they were before a second kernel shared them.
 __device__ __forceinline__ void rotate_pair(float& a, float& b, float c, float s) {
   const float x1 = a, x2 = b;
   a = __fmaf_rn(x1, c, -__fmul_rn(x2, s));
-  b = __fmaf_rn(x2, c, __fmul_rn(x1, s));
+  b = __fmaf_rn(x1, s, __fmul_rn(x2, c));
 }
-__device__ __forceinline__ float add_squares(float a, float b, float sum) { return __fmaf_rn(a, a, __fmaf_rn(b, b, sum)); }
+__device__ __forceinline__ float add_squares(float a, float b, float sum) { return __fadd_rn(sum, __fmaf_rn(a, a, __fmul_rn(b, b))); }
 
 // x * sigmoid(x).  The approximate division on purpose: the IEEE `/` takes a slow subroutine whenever the numerator
 // is zero or tiny, and zero rows are common here (padding rows of a graph bucket, rows of a partial token tile):

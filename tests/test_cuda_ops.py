@@ -470,6 +470,36 @@ def test_qk_norm_rope_store(ops, T, nq, nkv, bs):
     ops.check_status()
 
 
+def test_qk_norm_rope_store_rounds_in_a_fixed_order(ops):
+    """A head's bits: sums of squares as sum + (a^2 + b^2), an eight-element run per lane, then a tree over eight lanes; rotation as
+    x1 c - round(x2 s) and x1 s + round(x2 c).  Products of bf16 numbers are exact in fp32 and those with a table entry in 64 bits, so both
+    can be stated exactly; another order differs in a few of the 16 million elements (3 to 6 for the sums, over 120 for the rotation)."""
+    T, nq, nkv = 8192, 16, 8
+    torch.manual_seed(0)
+    qkv = _rand(T, (nq + 2 * nkv) * 128)
+    w = _rand(128, scale=0.2) + 1
+    table = ref.rope_table(4096, 128, 1e6, "cuda")
+    pos = torch.randint(0, 4096, (T,), dtype=torch.int32, device="cuda")
+    slots = torch.arange(T, dtype=torch.int32, device="cuda")
+    kc, vc = torch.zeros(32, nkv, 256, 128, dtype=BF, device="cuda"), torch.zeros(32, nkv, 256, 128, dtype=BF, device="cuda")
+    x = qkv.view(T, -1, 128)[:, :nq].float()
+    squares = (x * x).view(T, nq, 2, 8, 8)
+    sums = torch.zeros(T, nq, 8, device="cuda")
+    for e in range(8):
+        sums = sums + (squares[:, :, 0, :, e] + squares[:, :, 1, :, e])
+    for step in (1, 2, 4):
+        sums = sums + sums[..., [i ^ step for i in range(8)]]
+    normed = (x * torch.rsqrt(sums[..., :1] / 128 + 1e-6)).to(BF).float() * w.float()
+    got = ops.qk_norm_rope_store(qkv, w, w, 1e-6, table, pos, slots, kc, vc, nq, nkv, 128, do_rope=False)
+    assert torch.equal(got, normed.to(BF))
+    x1, x2 = x[..., :64].double(), x[..., 64:].double()
+    c, s = table[pos.long()][:, None].double().split(64, -1)
+    want = torch.cat([x1 * c - (x2 * s).float().double(), x1 * s + (x2 * c).float().double()], -1).float().to(BF)
+    got = ops.qk_norm_rope_store(qkv, None, None, 1e-6, table, pos, slots, kc, vc, nq, nkv, 128)
+    assert torch.equal(got, want)
+    ops.check_status()
+
+
 # ----------------------------------------------------------------------------- attention
 class _Batch:
     pass
