@@ -109,19 +109,22 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 
-// p = 2^(s * scale - m_ref) of 32 scores, as pairs of bf16 to tensor memory (16 columns); adds p to the two running sums.
-// Two scores per multiply-add and addition.  (A quarter or three eighths of the exponentials as polynomials on the multiply-add
+// p = 2^(s * scale - m_ref) of 32 scores, as pairs of bf16 to tensor memory (16 columns); adds p to the running sums, two sums to a register
+// pair: of the four pairs of eight scores, in the order of umma_probs_to_smem.  Two scores per multiply-add and addition.  (A quarter or three eighths of the exponentials as polynomials on the multiply-add
 // units instead: slower by 5 to 8 %, the one warp that is active per scheduler issues no faster.)
 __device__ __forceinline__ void pair_probs(const uint32_t* v, uint64_t scale2, uint64_t ref2, uint64_t (&sum)[2], uint32_t p_addr) {
   uint32_t pk[16];
 #pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    float p0, p1;
-    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), scale2, ref2), p0, p1);
-    p0 = ex2_approx(p0);
-    p1 = ex2_approx(p1);
-    sum[(i >> 1) & 1] = add_f32x2(sum[(i >> 1) & 1], pack_f32x2(p0, p1));
-    pk[i >> 1] = pack_bf16x2(p0, p1);
+  for (int i = 0; i < 32; i += 4) {
+    float p[4];
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+      unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(v[i + e]), __uint_as_float(v[i + e + 1])), scale2, ref2), p[e], p[e + 1]);
+      p[e] = ex2_approx(p[e]);
+      p[e + 1] = ex2_approx(p[e + 1]);
+      pk[(i + e) >> 1] = pack_bf16x2(p[e], p[e + 1]);
+    }
+    sum[(i >> 2) & 1] = add_f32x2(sum[(i >> 2) & 1], add_f32x2(pack_f32x2(p[0], p[2]), pack_f32x2(p[1], p[3])));
   }
   tmem_st_x16(p_addr, pk);
 }
@@ -422,9 +425,10 @@ __global__ void __launch_bounds__(kWThreads, 1) prefill_attn_pair_kernel(
           if (lane == 0) mbar_arrive(&p_full[2 * i + half]);
           if (half == 0) tmem_ld_wait();
         }
-        float l0, l1;
-        unpack_f32x2(add_f32x2(sum[0], sum[1]), l0, l1);
-        l_run += l0 + l1;
+        float l0, l1, l2, l3;
+        unpack_f32x2(sum[0], l0, l1);
+        unpack_f32x2(sum[1], l2, l3);
+        l_run += (l0 + l1) + (l2 + l3);
       }
       // all of O: wait for the last P V, normalise, store (rows that see nothing, and tiles without keys, are zero)
       if (ok && n > 0) ok = mbar_wait(&o_full[i], uses++ & 1, status);

@@ -52,7 +52,8 @@ __device__ __forceinline__ float umma_row_max(const uint32_t (&v)[kUN], int kbas
 }
 
 // p = 2^(s * scale - m_ref) for one row of a tile -> bf16 -> shared memory (K-major, 128-byte swizzle: 16-byte chunk
-// index ^ (row % 8)); returns the row sum, added up in the order of the two-tile kernel: a row's result does not depend on which one runs.
+// index ^ (row % 8)); returns the row sum, added up in the same order as in the two-tile kernel (four sums of pairs, pair i % 4): a row's
+// result does not depend on which one runs.
 template <bool kMasked>
 __device__ __forceinline__ float umma_probs_to_smem(const uint32_t (&v)[kUN], int kbase, int limit, float scale_log2, float m_ref,
                                                     uint8_t* p_row, int r) {
@@ -68,14 +69,13 @@ __device__ __forceinline__ float umma_probs_to_smem(const uint32_t (&v)[kUN], in
         p0 = kbase + c + i < limit ? p0 : 0.f;
         p1 = kbase + c + i + 1 < limit ? p1 : 0.f;
       }
-      ps[i & 2] += p0;
-      ps[(i & 2) + 1] += p1;
+      ps[i >> 1] += p0 + p1;
       pk[i >> 1] = pack_bf16x2(p0, p1);
     }
     const int chunk = (c & 63) >> 3;                   // 16-byte chunk (8 keys) within the 64-key half
     *reinterpret_cast<uint4*>(p_row + (c >> 6) * kUHalf + ((chunk ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
   }
-  return (ps[0] + ps[2]) + (ps[1] + ps[3]);
+  return (ps[0] + ps[1]) + (ps[2] + ps[3]);
 }
 
 // tm_q: 2-D view [T, nq * 128] of q, box 128 rows x 64 cols.  tm_k / tm_v: 2-D view [blocks * nkv * block_size, 128]

@@ -1,5 +1,7 @@
 """Every sm_100a kernel against the plain-PyTorch fp32 statement of the same op (ops/ref.py)."""
 
+import math
+
 import pytest
 import torch
 
@@ -709,6 +711,26 @@ def test_prefill_attention_two_tiles_per_cta(ops, q_lens, k_lens, nq, nkv, bs):
     for _ in range(2):
         got = ops.attention(q, kc, vc, b, 128 ** -0.5)
         _close(got, want, 2e-2, 2e-2)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("seqs,nq,nkv", [(1, 1, 1), (40, 4, 2), (40, 5, 5)])
+def test_prefill_attention_adds_row_sums_in_pairs(ops, seqs, nq, nkv):
+    """One query tile per CTA, and two (heads of a group, or rows).  The scores are whole numbers, so the weights are powers of two: 1 + 2^-9,
+    then 2^-18, then twice 2^-24 (the rest vanishes), and only the first value is 1.  Added pair by pair, the last two survive: the sum is
+    1 + 2^-9 + 2^-18 + 2^-23 and the result 2^-8 below 1.  One by one they are lost and the result, a tie in bf16, is 1."""
+    n = 128
+    q, kc, vc, b = _paged_case([n] * seqs, [n] * seqs, nq, nkv, 256)
+    b.is_prefill = True
+    exponents = torch.full((n,), -200.0)
+    for key, e in ((0, 0), (1, -9), (8, -18), (16, -24), (17, -24)):
+        exponents[key] = e
+    q.zero_(), kc.zero_(), vc.zero_()
+    q[:, :, 0] = 1
+    kc[:, :, :n, 0] = exponents.cuda().to(BF)
+    vc[:, :, 0] = 1
+    got = ops.attention(q, kc, vc, b, math.log(2)).view(seqs, n, nq * 128)          # times log2(e): a factor of exactly one
+    assert torch.all(got[:, 18:].float() == 1 - 2.0 ** -8)
     ops.check_status()
 
 
