@@ -24,7 +24,7 @@
 // of another warp is slow.  So it issues whole groups of products (one asm block each) and waits as rarely as possible.
 // The exponentials use a reference maximum that is only raised when the true row maximum has grown by more than 2^8 since it was set
 // (exact arithmetic either way: O and the row sum carry the same factor); only then do the softmax warps read O back,
-// scale it and store it again, which happens a few times per row instead of once per tile.  The end of an item (O is normalised and
+// scale it and store it again, which happens a few times per row instead of once per tile.  Each row decides for itself.  The end of an item (O is normalised and
 // stored) overlaps with the first scores of the next one.
 //
 // Items are dealt out from the last rows of the sequences (the most keys) to the first, forwards and backwards over the
@@ -392,10 +392,11 @@ __global__ void __launch_bounds__(kWThreads, 1) prefill_attn_pair_kernel(
         }
         if (j == 0) {
           m_ref = mt == -INFINITY ? 0.f : mt;            // O is not valid yet: nothing to rescale
-        } else if (__any_sync(0xffffffffu, mt - m_ref > 8.f)) {
-          // tcgen05.ld / .st are warp-wide: the whole warp rescales.  The commit behind s_full covered every earlier P V.
-          const float m_new = fmaxf(m_ref, mt);
-          const float alpha = exp2f(m_ref - m_new);      // 1 for rows whose maximum did not move
+        } else if (const bool grow = mt - m_ref > 8.f; __any_sync(0xffffffffu, grow)) {
+          // tcgen05.ld / .st are warp-wide: the whole warp rescales, rows whose maximum did not grow by exactly 1 (what a row gives does not
+          // depend on its neighbours).  The commit behind s_full covered every earlier P V.
+          const float m_new = grow ? mt : m_ref;
+          const float alpha = exp2f(m_ref - m_new);
 #pragma unroll 1
           for (int c = 0; c < kWD; c += 32) {
             uint32_t o[32];

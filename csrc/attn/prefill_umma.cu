@@ -250,8 +250,8 @@ __global__ void __launch_bounds__(kUThreads, 1) prefill_attn_umma_kernel(
           ok = mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, status);            // every earlier P V has landed in O
           if (!ok) break;
           tcgen05_fence_after();
-          const float m_new = fmaxf(m_ref, mt);
-          const float alpha = exp2f(m_ref - m_new);      // 1 for rows whose maximum did not move
+          const float m_new = grow ? mt : m_ref;         // row by row: what a row gives does not depend on its neighbours
+          const float alpha = exp2f(m_ref - m_new);      // exactly 1 for the others
 #pragma unroll 1
           for (int c = 0; c < kUD; c += 32) {
             uint32_t o[32];

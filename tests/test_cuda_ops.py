@@ -734,21 +734,57 @@ def test_prefill_attention_adds_row_sums_in_pairs(ops, seqs, nq, nkv):
     ops.check_status()
 
 
-def test_prefill_attention_does_not_depend_on_the_batch(ops):
-    """A sequence alone (one query tile per CTA) and the same one among others (two): the same bits, so a prompt computed in portions or beside
-    others gives the tokens it gives by itself."""
-    lens = [1000, 333, 129, 64] + [300] * 8
-    q, kc, vc, b = _paged_case(lens, lens, 16, 8, 256, seed=5)
+def _growing_keys(q, kc, b, nq, nkv, bs):
+    """Adds a direction to q and k along which the keys grow from one 128-key tile to the next: the maxima of a part of the rows (a third of
+    them, of different heads) jump by 10 to 40 in the exponent of 2 again and again, others by less than the 8 from which O is rescaled, a third not."""
+    u = torch.nn.functional.normalize(torch.randn(128, device="cuda"), dim=0)
+    strength = torch.tensor([0.0, 1.0, 6.0], device="cuda")[torch.randint(0, 3, q.shape[:2], device="cuda")] * (1 + torch.rand(q.shape[:2], device="cuda"))
+    q += (strength[..., None] * u * 128 ** 0.5).to(BF)
+    for s in range(b.num_seqs):
+        for i in range(-(-int(b.context_lens[s]) // bs)):
+            tile = (i * bs + torch.arange(bs, device="cuda")) // 128
+            kc[b.block_tables[s, i]] += (1.5 * tile[:, None] * u).to(BF)
+
+
+@pytest.mark.parametrize("q_lens,k_lens,nq,nkv,bs", [
+    ([900], [900], 4, 2, 256), ([100, 300], [1400, 800], 3, 1, 128),                                     # one query tile per CTA
+    ([1000, 300, 77], [1000, 300, 77], 32, 8, 256), ([200] * 6, [1224] * 6, 16, 8, 256),                 # two: heads of a group
+    ([700, 129, 300], [700, 1153, 300], 27, 9, 256), ([400] * 5, [900] * 5, 10, 10, 512),                # two: rows of a head
+])
+def test_prefill_attention_with_growing_maxima(ops, q_lens, k_lens, nq, nkv, bs):
+    """O is read back, scaled and stored between two products with V (tolerance of the tests above: bf16 operands and weights)."""
+    q, kc, vc, b = _paged_case(q_lens, k_lens, nq, nkv, bs, seed=3)
     b.is_prefill = True
+    _growing_keys(q, kc, b, nq, nkv, bs)
+    want = ref.attention(q, kc, vc, b.cu_seqlens_q, b.context_lens, b.block_tables, 128 ** -0.5, b.num_seqs)
+    got = ops.attention(q, kc, vc, b, 128 ** -0.5)
+    _close(got, want, 2e-2, 2e-2)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("grow", [False, True])
+@pytest.mark.parametrize("nq,nkv", [(16, 8), (24, 8)])
+def test_prefill_attention_does_not_depend_on_the_batch(ops, nq, nkv, grow):
+    """A sequence alone (one query tile per CTA), the same one among others (two), and computed in portions that are no multiples of a tile:
+    the same bits, so a prompt computed in portions or beside others gives the tokens it gives by itself.  Also where maxima grow, and with
+    another sequence's queries behind the last rows of a tile."""
+    lens = [1000, 333, 129, 64] + [300] * 8
+    q, kc, vc, b = _paged_case(lens, lens, nq, nkv, 256, seed=5)
+    b.is_prefill = True
+    if grow:
+        _growing_keys(q, kc, b, nq, nkv, 256)
     whole = ops.attention(q, kc, vc, b, 128 ** -0.5)
     at = 0
     for i, n in enumerate(lens[:4]):
-        one = _Batch()
-        one.is_prefill, one.num_seqs, one.padded_seqs, one.table_width = True, 1, 1, b.table_width
-        one.cu_seqlens_q = torch.tensor([0, n], dtype=torch.int32, device="cuda")
-        one.context_lens, one.block_tables = b.context_lens[i:i + 1].contiguous(), b.block_tables[i:i + 1].contiguous()
-        one.max_seqlen_q = one.max_seqlen_k = n
-        assert torch.equal(ops.attention(q[at:at + n].contiguous(), kc, vc, one, 128 ** -0.5), whole[at:at + n])
+        for first, last in [(0, n), (0, n // 3), (n // 3, n - n // 4), (n - n // 4, n)]:
+            one = _Batch()
+            one.is_prefill, one.num_seqs, one.padded_seqs, one.table_width = True, 1, 1, b.table_width
+            one.cu_seqlens_q = torch.tensor([0, last - first], dtype=torch.int32, device="cuda")
+            one.context_lens = torch.tensor([last], dtype=torch.int32, device="cuda")
+            one.block_tables = b.block_tables[i:i + 1].contiguous()
+            one.max_seqlen_q, one.max_seqlen_k = last - first, last
+            rows = slice(at + first, at + last)
+            assert torch.equal(ops.attention(q[rows].contiguous(), kc, vc, one, 128 ** -0.5), whole[rows]), (i, first, last)
         at += n
     ops.check_status()
 
