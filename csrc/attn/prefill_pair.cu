@@ -31,7 +31,7 @@
 // CTAs in turn, so that long and short ones add up alike; every warp walks the same list by itself from the lengths.
 //
 // The query rows of a sequence are its LAST q_len positions; with a cached prefix the causal mask is aligned to the
-// bottom-right corner: query row i sees keys 0 .. (k_len - q_len + i).  All waits are bounded (ptx.cuh).
+// bottom-right corner: query row i sees keys 0 .. (k_len - q_len + i).  scale > 0 (hidden scores are -inf).  All waits are bounded (ptx.cuh).
 #include "../include/launch.cuh"
 #include "../include/ptx.cuh"
 

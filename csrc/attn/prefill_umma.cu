@@ -339,7 +339,8 @@ extern "C" int forge_prefill_attention_umma(const void* q, const void* kc, const
   // CTA (prefill_pair.cu).  Measured, one against two: 1 x 1000 tokens of 16 heads (128 tiles) 22.6 / 31.7 us, 4 x 700 of 5 heads (120) 20.5 / 25.6;
   // 12 x 100 of 16 heads (192) 20.6 / 16.4, 1 x 700 of 32 heads (192) 28.7 / 24.6, 1 x 1300 of 16 heads (176) 35.6 / 35.6, 2 x 513 of 32 heads 34.8 / 24.6.
   const long long tiles = std::min<long long>(static_cast<long long>(num_seqs) * ((max_q + kUM - 1) / kUM), T / kUM + num_seqs) * nq;
-  if (tiles > device_sm_count())
+  // A scale of zero or less stays here whatever the number of tiles: the pair kernel hides a key by a score of -inf, which needs a positive factor.
+  if (tiles > device_sm_count() && scale_log2 > 0.f)
     return launch_prefill_attn_pair(tm_q, tm_k, tm_v, cu_q, lens, bt, out, T, num_seqs, max_q, nq, nkv, block_size, table_width, num_blocks, scale_log2,
                                     status, stream);
   constexpr int smem = (1 + 2 * kUStages + 2) * kUTile + 256 + 1024;

@@ -734,6 +734,17 @@ def test_prefill_attention_adds_row_sums_in_pairs(ops, seqs, nq, nkv):
     ops.check_status()
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.05])
+@pytest.mark.parametrize("q_lens,k_lens", [([300], [300]), ([300] * 12, [300] * 6 + [684] * 6)])
+def test_prefill_attention_with_a_scale_that_is_not_positive(ops, q_lens, k_lens, scale):
+    """Zero (every visible key counts the same) and less, with few query tiles and with many (each row sees a key of each of its tiles)."""
+    q, kc, vc, b = _paged_case(q_lens, k_lens, 8, 4, 256, seed=6)
+    b.is_prefill = True
+    want = ref.attention(q, kc, vc, b.cu_seqlens_q, b.context_lens, b.block_tables, scale, b.num_seqs)
+    _close(ops.attention(q, kc, vc, b, scale), want, 2e-2, 2e-2)
+    ops.check_status()
+
+
 def _growing_keys(q, kc, b, nq, nkv, bs):
     """Adds a direction to q and k along which the keys grow from one 128-key tile to the next: the maxima of a part of the rows (a third of
     them, of different heads) jump by 10 to 40 in the exponent of 2 again and again, others by less than the 8 from which O is rescaled, a third not."""
