@@ -283,7 +283,10 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
       } else {
         const size_t p = (static_cast<size_t>(it.b) * nq + qh0 + g) * max_chunks + it.c;
         part_o[p * kD + d] = ov;
-        if (d == 0) *reinterpret_cast<float2*>(part_ml + p * 2) = make_float2(M, L);
+        if (d == 0) {
+          part_ml[p * 2] = M;
+          part_ml[p * 2 + 1] = L;
+        }
       }
     }
     named_barrier_sync(1, 128);                         // s_acc and s_q are the next item's

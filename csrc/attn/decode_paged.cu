@@ -156,6 +156,11 @@ __global__ void __launch_bounds__(kDecThreads, decode_ctas_per_sm(G)) decode_att
   }
 }
 
+// A (max, sum) pair; a caller's scratch may begin at any float, so the pair is read at once only where its address allows.
+__device__ __forceinline__ float2 combine_load_pair(const float* __restrict__ ml, size_t i, bool aligned) {
+  return aligned ? reinterpret_cast<const float2*>(ml)[i] : make_float2(ml[2 * i], ml[2 * i + 1]);
+}
+
 // Merge the per-chunk partials of sequences that span more than one chunk.  The (max, sum) pairs are read by all threads at once and the
 // partial rows eight at a time: with one after another the merge of 47 chunks took 8.7 us, longer than it took to make half of them.
 __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
@@ -170,13 +175,14 @@ __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restr
   const int n = (len + chunk - 1) / chunk;
   if (n <= 1) return;
   const size_t base = (static_cast<size_t>(b) * nq + qh) * max_chunks;
-  const float2* ml = reinterpret_cast<const float2*>(part_ml) + base;
+  const float* ml = part_ml + base * 2;
+  const bool aligned = (reinterpret_cast<uintptr_t>(part_ml) & 7) == 0;
   if (n <= 8) {                                          // everything at once, nothing between threads
     float2 x[8];
     float v[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      x[c] = c < n ? ml[c] : make_float2(-INFINITY, 0.f);
+      x[c] = c < n ? combine_load_pair(ml, c, aligned) : make_float2(-INFINITY, 0.f);
       v[c] = c < n ? part_o[(base + c) * kD + d] : 0.f;
     }
     float M = x[0].x, L = 0.f, O = 0.f;
@@ -191,9 +197,9 @@ __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restr
     out[(static_cast<size_t>(b) * nq + qh) * kD + d] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
     return;
   }
-  const float2 first = d < n ? ml[d] : make_float2(-INFINITY, 0.f);
+  const float2 first = d < n ? combine_load_pair(ml, d, aligned) : make_float2(-INFINITY, 0.f);
   float M = first.x;
-  for (int c = d + kD; c < n; c += kD) M = fmaxf(M, ml[c].x);
+  for (int c = d + kD; c < n; c += kD) M = fmaxf(M, ml[2 * c]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   if ((d & 31) == 0) s_max[d >> 5] = M;
@@ -201,7 +207,7 @@ __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restr
   M = fmaxf(fmaxf(s_max[0], s_max[1]), fmaxf(s_max[2], s_max[3]));
   float L = 0.f, O = 0.f;
   for (int c0 = 0; c0 < n; c0 += kD) {
-    const float2 x = c0 == 0 ? first : c0 + d < n ? ml[c0 + d] : make_float2(-INFINITY, 0.f);
+    const float2 x = c0 == 0 ? first : c0 + d < n ? combine_load_pair(ml, c0 + d, aligned) : make_float2(-INFINITY, 0.f);
     if (c0 > 0) __syncthreads();
     s_w[d] = x.y * exp2f(x.x - M);
     __syncthreads();

@@ -658,6 +658,21 @@ def test_decode_attention_chunks_on_tensor_cores(ops, k_lens, nq, nkv, bs, chunk
     ops.check_status()
 
 
+@pytest.mark.parametrize("k_lens,nq,nkv", [([700, 5, 300], 16, 8), ([700, 5, 300], 32, 8), ([1500], 8, 8)])
+def test_decode_attention_with_a_scratch_that_begins_anywhere(ops, k_lens, nq, nkv):
+    """Views at an odd number of floats from an aligned address, few and more than eight chunks to merge."""
+    q, kc, vc, b = _paged_case([1] * len(k_lens), k_lens, nq, nkv, 256, seed=8)
+    want = ref.attention(q, kc, vc, b.cu_seqlens_q, b.context_lens, b.block_tables, 128 ** -0.5, b.num_seqs)
+    for chunk in (64, 256):
+        max_chunks = -(-max(k_lens) // chunk)
+        need = len(k_lens) * nq * max_chunks
+        part_o, part_ml = torch.empty(need * 128 + 1, device="cuda")[1:], torch.empty(need * 2 + 1, device="cuda")[1:]
+        got = torch.empty(len(k_lens), nq * 128, dtype=BF, device="cuda")
+        ops.C.decode_attention(q, kc, vc, b.block_tables, b.context_lens, got, part_o, part_ml, chunk, max_chunks, 128 ** -0.5, ops.status)
+        _close(got, want.view_as(got), 2e-2, 2e-2)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("batch,lo,hi,nq,nkv", [(64, 100, 1500, 16, 8), (200, 1, 700, 16, 8), (300, 3000, 3100, 8, 2), (7, 1, 4000, 32, 8),
                                                 (70, 100, 2500, 64, 8)])
 def test_decode_attention_flat_partition_many_sequences(ops, batch, lo, hi, nq, nkv, monkeypatch):
