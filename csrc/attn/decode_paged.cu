@@ -276,15 +276,16 @@ static int decode_chunked_impl(const void* q, const void* kc, const void* vc, co
   const int tile = block_size < 64 ? block_size : 64;
   if (chunk % tile != 0 || max_chunks < 1) return -1;
   if (max_chunks > 1 && (part_o == nullptr || part_ml == nullptr)) return -1;
+  if (((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) != 0) return -1;     // bulk and tensor copies alike need 16 bytes
   const int group = nq / nkv;
   const int G = decode_group_slice(group);
   const float sl2 = scale * 1.4426950408889634f;
   // Very few sequences: at most 24 chunks each, more of them cost the merge more than they save (3001 tokens of 32 / 8 heads: 47 chunks 15.5 us, 24: 13.3).
   const int parts = B * nkv < 32 ? std::min(max_chunks, 24) : max_chunks;
-  // Groups of 4 to 8 heads, cache blocks of 64 tokens and more: on the tensor cores (decode_chunks.cu); TMA wants 16-byte rows.  With two heads per
+  // Groups of 4 to 8 heads, cache blocks of 64 tokens and more: on the tensor cores (decode_chunks.cu).  With two heads per
   // KV head the CUDA cores keep up with the stream and their kernel starts faster (2 sequences 12.0 us against 13.8, 40: 44 against 53); with four
   // they do not (13 sequences: 31.7 against 22.4).
-  if (tile == 64 && group >= 4 && group <= 8 && ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0) {
+  if (tile == 64 && group >= 4 && group <= 8) {
     const int rc = launch_decode_chunks(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, chunk, max_chunks, parts, sl2,
                                         status, stream, fuse);
     if (rc != 0 || max_chunks <= 1) return rc;

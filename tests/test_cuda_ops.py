@@ -537,6 +537,7 @@ def _paged_case(q_lens, k_lens, nq, nkv, bs, seed=0):
 @pytest.mark.parametrize("k_lens,nq,nkv,bs", [
     ([1], 16, 8, 256), ([5, 300, 64, 1000], 16, 8, 256), ([17, 33, 250], 8, 2, 16), ([700, 2011, 129], 32, 8, 256),
     ([40, 90], 8, 8, 32), ([513, 77], 8, 1, 64), ([300, 1000, 70, 2], 40, 8, 256), ([129, 640, 33], 64, 8, 256), ([50, 400], 6, 2, 64), ([700, 2011, 129], 8, 1, 256),
+    ([300, 65, 2], 10, 1, 64), ([700, 129], 24, 2, 256), ([500, 1], 15, 1, 128), ([64, 513], 32, 2, 256),          # groups over 8: slices of 5 and 4 heads
 ])
 def test_decode_attention(ops, k_lens, nq, nkv, bs, mode, monkeypatch):
     monkeypatch.setattr(ops, "decode_attention_mode", mode)
@@ -585,7 +586,7 @@ def test_decode_attention_padding_rows(ops, mode, monkeypatch):
 @pytest.mark.parametrize("k_lens,nq,nkv,bs", [
     ([1, 2, 64, 65, 300, 1000, 0, 256, 257, 512], 16, 8, 256), ([17, 33, 250, 16, 1], 8, 2, 16), ([700, 2011, 129, 128], 32, 8, 256),
     ([40, 90, 64], 8, 8, 32), ([513, 77], 8, 1, 64), (list(range(1, 140, 3)), 16, 8, 128), ([300, 1000, 70, 2], 40, 8, 256),
-    ([129, 640, 33], 64, 8, 256),
+    ([129, 640, 33], 64, 8, 256), ([300, 0, 64], 10, 1, 64), ([129, 500], 32, 2, 256),
 ])
 def test_decode_attention_from_raw_qkv(ops, k_lens, nq, nkv, bs, mode, monkeypatch):
     """q/k-norm + rotation + KV store inside the attention kernel == qk_norm_rope_store followed by attention:
@@ -670,6 +671,18 @@ def test_decode_attention_with_a_scratch_that_begins_anywhere(ops, k_lens, nq, n
         got = torch.empty(len(k_lens), nq * 128, dtype=BF, device="cuda")
         ops.C.decode_attention(q, kc, vc, b.block_tables, b.context_lens, got, part_o, part_ml, chunk, max_chunks, 128 ** -0.5, ops.status)
         _close(got, want.view_as(got), 2e-2, 2e-2)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("nq,nkv", [(16, 8), (32, 8)])
+def test_decode_attention_refuses_a_cache_that_is_not_aligned(ops, nq, nkv):
+    """Every kernel copies cache rows 16 bytes at a time; a cache that begins elsewhere is an error on the host."""
+    q, kc, vc, b = _paged_case([1], [50], nq, nkv, 64)
+    odd = torch.zeros(vc.numel() + 4, dtype=BF, device="cuda")[4:].view(vc.shape)
+    got = torch.empty(1, nq * 128, dtype=BF, device="cuda")
+    for k, v in ((kc, odd), (odd, vc)):
+        with pytest.raises(RuntimeError):
+            ops.C.decode_attention(q, k, v, b.block_tables, b.context_lens, got, None, None, 128, 1, 128 ** -0.5, ops.status)
     ops.check_status()
 
 
