@@ -4,8 +4,10 @@
 // read on the device, so the launch fits a CUDA graph whatever they become.  A CTA streams tiles of 64 tokens of K and V (2-D TMA boxes
 // of 64 rows x 64 dims with the 128-byte swizzle, a ring of two stages that never drains across items) and its four consumer warps take
 // 16 tokens of each tile: S = Q K^T and O += P V as mma.sync m16n8k16 with fp32 sums.  The heads of the group fill rows 0..7 of the
-// query tile.  The weights keep 16 bits of their mantissa: P = hi + lo, two bf16 numbers; hi fills rows 0..7 of the second product
-// and lo rows 8..15, which would be empty.  A sequence of one chunk is finished here, others leave partials for the merge kernel.
+// query tile.  The weights keep all 24 bits of their mantissa: P = hi + mid + lo, three bf16 numbers of 8 bits each, cut off and not rounded, so
+// that none is negative and their sum is P exactly.  hi fills rows 0..7 of the second product and mid rows 8..15, which would be empty.  With
+// four heads lo has rows 4..7, whose queries are those of rows 0..3 once more; with more it takes a product of its own.  A sequence of one chunk is
+// finished here, others leave partials for the merge kernel.
 //
 // What bounds it is latency (length -> block table -> keys -> scores -> sums), and from about ten sequences the stream of the cache: three
 // CTAs per SM with 64 KB on their way each.  The dot products on the CUDA cores, which this replaces for cache blocks of 64 tokens and more,
@@ -31,6 +33,10 @@ __host__ __device__ constexpr int ck_ctas_per_sm(int G) { return G > 4 ? 2 : 3; 
 __device__ __forceinline__ uint32_t ck_addr(uint32_t tile, int r, int piece) {
   return tile + (piece >> 3) * kCkBox + r * 128 + (((piece & 7) ^ (r & 7)) << 4);
 }
+
+// The parts of a weight: the upper 16 bits of p, of what is left, and of what is left then (at most 8 bits: exact).
+__device__ __forceinline__ float ck_upper(float p) { return __uint_as_float(__float_as_uint(p) & 0xFFFF0000u); }
+__device__ __forceinline__ uint32_t ck_pack_upper(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
 
 struct ChunkItem {
   int b, c, kvh, len, chunk;
@@ -94,7 +100,8 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* s_acc = reinterpret_cast<float*>(smem + kCkStages * 2 * kCkTileBytes);          // merge area
   __nv_bfloat16* s_q = reinterpret_cast<__nv_bfloat16*>(s_acc + decode_merge_floats(G)); // [G][128]
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(s_q + G * kD);
+  uint4* s_new = reinterpret_cast<uint4*>(s_q + G * kD); // the newest token: 16 pieces of its key, 16 of its value
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(s_new + 32);
   uint64_t* empty_bar = full_bar + kCkStages;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -147,7 +154,10 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
   for (int b = blockIdx.x; b < B; b += gridDim.x)       // padding rows (length 0): defined output
     if (context_lens[b] <= 0)
       for (int i = threadIdx.x; i < nq * kD; i += 128) out[static_cast<size_t>(b) * nq * kD + i] = __float2bfloat16_rn(0.f);
-  const int row = lane >> 2, quad = lane & 3;           // fragment coordinates: head of the group, column pair
+  constexpr bool kLoInRows = G <= 4;                    // rows 4..7 are free for the third part of the weights
+  const int row = lane >> 2, quad = lane & 3;           // fragment coordinates: row of the query tile, column pair
+  const int head = kLoInRows ? row & 3 : row;           // head of the group
+  const bool lo_row = kLoInRows && row >= 4;
   const int mat = lane >> 3, mrow = lane & 7;           // ldmatrix: this lane supplies row `mrow` of matrix `mat`
   int n = 0;
   bool ok = true;                                       // once a wait has run out none is made any more, but every barrier still is
@@ -157,8 +167,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
     // the newest token (position len - 1) is not in the cache yet: the warp that owns its row of its tile prepares it now
     const int newest = it.len - 1, row_new = newest % kCkTile;
     const bool owner = fuse.qkv != nullptr && newest >= begin && newest < end && warp == row_new / 16;
-    DecodeNewToken fresh = {};
-    uint32_t qa[8][2];                                  // rows 0..G-1 = the heads of the group, the others zero; 8 steps of 16 dims
+    uint32_t qa[8][2];                                  // rows 0..G-1 = the heads of the group, the others zero (G = 4: again the heads); 8 steps of 16 dims
     if (fuse.qkv != nullptr) {
       const float* cs = fuse.rope != nullptr ? fuse.rope + static_cast<size_t>(min(max(newest, 0), fuse.rope_rows - 1)) * kD : nullptr;
       for (int g = warp; g < G; g += 4) {
@@ -171,19 +180,26 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
               make_uint4(pack_bf16x2(x[8], x[9]), pack_bf16x2(x[10], x[11]), pack_bf16x2(x[12], x[13]), pack_bf16x2(x[14], x[15]));
         }
       }
-      if (owner) fresh = decode_new_token(fuse, it.b, it.kvh, nq, nkv, it.len, lane);
+      if (owner) {                                      // kept in shared memory: ten registers less across the loop
+        const DecodeNewToken fresh = decode_new_token(fuse, it.b, it.kvh, nq, nkv, it.len, lane);
+        if (lane < 8) {
+          s_new[lane] = fresh.k_lo;
+          s_new[8 + lane] = fresh.k_hi;
+        }
+        reinterpret_cast<uint2*>(s_new + 16)[lane] = fresh.v;
+      }
       named_barrier_sync(1, 128);
     }
     {
-      const __nv_bfloat16* qp = (fuse.qkv != nullptr ? s_q : q + (static_cast<size_t>(it.b) * nq + qh0) * kD) + row * kD + 2 * quad;
+      const __nv_bfloat16* qp = (fuse.qkv != nullptr ? s_q : q + (static_cast<size_t>(it.b) * nq + qh0) * kD) + head * kD + 2 * quad;
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
-        qa[kk][0] = row < G ? *reinterpret_cast<const uint32_t*>(qp + kk * 16) : 0u;
-        qa[kk][1] = row < G ? *reinterpret_cast<const uint32_t*>(qp + kk * 16 + 8) : 0u;
+        qa[kk][0] = head < G ? *reinterpret_cast<const uint32_t*>(qp + kk * 16) : 0u;
+        qa[kk][1] = head < G ? *reinterpret_cast<const uint32_t*>(qp + kk * 16 + 8) : 0u;
       }
     }
-    float m_run = -INFINITY, l_run = 0.f;               // of head `row`; l is this lane's share until the end
-    float o[16][4];                                     // [..][0, 1]: sums of hi V, [2, 3]: of lo V, of the same head and dims
+    float m_run = -INFINITY, l_run = 0.f;               // of `head`; l is this lane's share until the end
+    float o[16][4];                                     // [..][0, 1]: sums of hi V (lo_row: of lo V), [2, 3]: of mid V (and of lo V), same head and dims
 #pragma unroll
     for (int nb = 0; nb < 16; ++nb) o[nb][0] = o[nb][1] = o[nb][2] = o[nb][3] = 0.f;
     for (int tok0 = begin; tok0 < end; tok0 += kCkTile, ++n) {
@@ -196,66 +212,85 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
         const bool to_cache = blk >= 0 && blk < num_blocks;
         if (!to_cache) blk = 0;
         const size_t off = ((static_cast<size_t>(blk) * nkv + it.kvh) * block_size + newest % block_size) * kD;
-        if (lane < 8) {
-          *reinterpret_cast<uint4*>(stg + (ck_addr(Ks, row_new, lane) - Ks)) = fresh.k_lo;
-          *reinterpret_cast<uint4*>(stg + (ck_addr(Ks, row_new, 8 + lane) - Ks)) = fresh.k_hi;
-          if (to_cache) {
-            *reinterpret_cast<uint4*>(k_cache + off + 8 * lane) = fresh.k_lo;
-            *reinterpret_cast<uint4*>(k_cache + off + 64 + 8 * lane) = fresh.k_hi;
-          }
-        }
-        *reinterpret_cast<uint2*>(stg + (ck_addr(Vs, row_new, lane >> 1) - Ks) + (lane & 1) * 8) = fresh.v;
-        if (to_cache) *reinterpret_cast<uint2*>(v_cache + off + lane * 4) = fresh.v;
+        const uint4 piece = s_new[lane];
+        *reinterpret_cast<uint4*>(stg + (ck_addr(lane < 16 ? Ks : Vs, row_new, lane & 15) - Ks)) = piece;
+        if (to_cache) *reinterpret_cast<uint4*>((lane < 16 ? k_cache : v_cache) + off + 8 * (lane & 15)) = piece;
         fence_proxy_async_smem();                       // a later copy into this stage comes after these writes
         __syncwarp();
       }
       const int r0 = warp * 16;
-      float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      // A product from zero for every 16 dims, added up here, pairs first: a sum that is carried on from product to product is cut off and not
+      // rounded at each of them.
+      float sc[2][2], part[2][3][2];                    // part: sums of one, two and four products
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
         uint32_t kb[4];
         ldsm_x4(ck_addr(Ks, r0 + (mat >> 1) * 8 + mrow, 2 * kk + (mat & 1)), kb);
         const uint32_t a[4] = {qa[kk][0], 0u, qa[kk][1], 0u};
-        mma16816(sc[0], a, kb[0], kb[1]);
-        mma16816(sc[1], a, kb[2], kb[3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float c[4] = {0.f, 0.f, 0.f, 0.f};
+          mma16816(c, a, kb[2 * j], kb[2 * j + 1]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float sum = c[e];
+            if (kk % 2 == 1) sum = part[j][0][e] + sum;
+            if (kk % 4 == 3) sum = part[j][1][e] + sum;
+            if (kk == 7) sc[j][e] = part[j][2][e] + sum;
+            else part[j][kk % 2 == 0 ? 0 : kk % 4 == 1 ? 1 : 2][e] = sum;
+          }
+        }
       }
-      // this lane: head `row`, tokens r0 + j * 8 + 2 * quad + {0, 1} of the tile
+      // this lane: `head`, tokens r0 + j * 8 + 2 * quad + {0, 1} of the tile
       const int valid = end - tok0;
       float mt = -INFINITY;
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          sc[j][e] = r0 + j * 8 + 2 * quad + e < valid ? sc[j][e] * scale_log2 : -INFINITY;
-          mt = fmaxf(mt, sc[j][e]);
-        }
+        for (int e = 0; e < 2; ++e)
+          if (r0 + j * 8 + 2 * quad + e < valid) mt = fmaxf(mt, sc[j][e] * scale_log2);
       mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 1));
       mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 2));
       const float m_new = fmaxf(m_run, mt);
       const float m_use = m_new == -INFINITY ? 0.f : m_new;
       const float alpha = exp2f(m_run - m_use);
-      float p[2][2], hi[2][2];
+      float p[2][2], mid[2][2], lo[2][2];
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          p[j][e] = exp2f(sc[j][e] - m_use);
-          hi[j][e] = decode_bf16_round(p[j][e]);
+          p[j][e] = r0 + j * 8 + 2 * quad + e < valid ? exp2f(fmaf(sc[j][e], scale_log2, -m_use)) : 0.f;
+          mid[j][e] = p[j][e] - ck_upper(p[j][e]);
+          lo[j][e] = mid[j][e] - ck_upper(mid[j][e]);
         }
-      l_run = l_run * alpha + (p[0][0] + p[0][1] + p[1][0] + p[1][1]);
+      l_run = fmaf(l_run, alpha, (p[0][0] + p[0][1]) + (p[1][0] + p[1][1]));
       m_run = m_new;
+      uint32_t pa[4], pl[2];
 #pragma unroll
-      for (int nb = 0; nb < 16; ++nb)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[nb][e] *= alpha;
-      const uint32_t pa[4] = {pack_bf16x2(hi[0][0], hi[0][1]), pack_bf16x2(p[0][0] - hi[0][0], p[0][1] - hi[0][1]),
-                              pack_bf16x2(hi[1][0], hi[1][1]), pack_bf16x2(p[1][0] - hi[1][0], p[1][1] - hi[1][1])};
+      for (int j = 0; j < 2; ++j) {
+        pa[2 * j] = ck_pack_upper(p[j][0], p[j][1]);
+        pa[2 * j + 1] = ck_pack_upper(mid[j][0], mid[j][1]);
+        pl[j] = ck_pack_upper(lo[j][0], lo[j][1]);
+        if (lo_row) {
+          pa[2 * j] = pl[j];
+          pa[2 * j + 1] = 0u;
+        }
+      }
 #pragma unroll
       for (int dd = 0; dd < 8; ++dd) {
         uint32_t vb[4];
         ldsm_x4_trans(ck_addr(Vs, r0 + (mat & 1) * 8 + mrow, 2 * dd + (mat >> 1)), vb);
-        mma16816(o[2 * dd], pa, vb[0], vb[1]);
-        mma16816(o[2 * dd + 1], pa, vb[2], vb[3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float c[4] = {0.f, 0.f, 0.f, 0.f};
+          mma16816(c, pa, vb[2 * j], vb[2 * j + 1]);
+          if constexpr (!kLoInRows) {
+            const uint32_t pb[4] = {0u, pl[0], 0u, pl[1]};
+            mma16816(c, pb, vb[2 * j], vb[2 * j + 1]);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[2 * dd + j][e] = fmaf(o[2 * dd + j][e], alpha, c[e]);
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty_bar[s]);
@@ -263,6 +298,12 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
     // ---- publish the warp's state in the layout decode_merged reads, merge, store
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+    if constexpr (kLoInRows) {
+#pragma unroll
+      for (int nb = 0; nb < 16; ++nb)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) o[nb][2 + e] += __shfl_xor_sync(0xffffffffu, o[nb][e], 16);
+    }
     if (row < G) {
       float* dst = s_acc + (warp * G + row) * kD + 2 * quad;
 #pragma unroll
@@ -299,7 +340,7 @@ template <int G>
 static int launch_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
                          int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk, int max_chunks, int parts, float scale_log2, unsigned* status,
                          cudaStream_t stream, const DecodeFuse& fuse) {
-  constexpr int smem = kCkStages * 2 * kCkTileBytes + decode_merge_floats(G) * 4 + G * kD * 2 + 2 * kCkStages * 8 + 1024;
+  constexpr int smem = kCkStages * 2 * kCkTileBytes + decode_merge_floats(G) * 4 + G * kD * 2 + 512 + 2 * kCkStages * 8 + 1024;
   static_assert(ck_ctas_per_sm(G) * (smem + 1024) <= 228 * 1024, "CTAs per SM");
   auto kern = decode_attn_chunk_kernel<G>;
   FORGE_ENSURE_DYN_SMEM(kern, smem);
