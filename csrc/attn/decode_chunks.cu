@@ -89,6 +89,36 @@ __device__ __forceinline__ bool chunk_item(const int* __restrict__ lens, int B, 
   return false;
 }
 
+// Sums of a warp that came out as NaN, once more with whole weights, one after the other.  An infinite value under a positive weight is an
+// infinite sum, but a part of the weight can be zero, and zero times infinity is not a number; what is NaN here too stays one.  q_rows: the
+// heads' queries (shared or global memory); o, m: the warp's sums and maxima.  Executed by a whole warp, rarely, hence not inlined.
+__device__ __noinline__ void ck_repair_sums(float* o, const float* m, int heads, const __nv_bfloat16* q_rows, const __nv_bfloat16* k_cache,
+                                            const __nv_bfloat16* v_cache, const int* table, int begin, int end, int kvh, int nkv, int block_size,
+                                            int num_blocks, float scale_log2, int lane) {
+  for (int g = 0; g < heads; ++g) {
+    float q[4], sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) q[e] = __bfloat162float(q_rows[g * kD + 4 * lane + e]);
+    const float m_use = m[g] == -INFINITY ? 0.f : m[g];
+    for (int tok0 = begin; tok0 < end; tok0 += kCkTile)
+      for (int tok = tok0; tok < min(tok0 + 16, end); ++tok) {
+        const int blk = table[tok / block_size];
+        const size_t off = ((static_cast<size_t>(blk >= 0 && blk < num_blocks ? blk : 0) * nkv + kvh) * block_size + tok % block_size) * kD + 4 * lane;
+        float d = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d = fmaf(q[e], __bfloat162float(k_cache[off + e]), d);
+#pragma unroll
+        for (int i = 16; i > 0; i >>= 1) d += __shfl_xor_sync(0xffffffffu, d, i);
+        const float p = exp2f(d * scale_log2 - m_use);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[e] = fmaf(p, __bfloat162float(v_cache[off + e]), sum[e]);
+      }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (isnan(o[g * kD + 4 * lane + e])) o[g * kD + 4 * lane + e] = sum[e];
+  }
+}
+
 template <int G>
 __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_chunk_kernel(
     const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __nv_bfloat16* __restrict__ q,
@@ -304,14 +334,25 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
 #pragma unroll
         for (int e = 0; e < 2; ++e) o[nb][2 + e] += __shfl_xor_sync(0xffffffffu, o[nb][e], 16);
     }
+    bool repair = false;
     if (row < G) {
       float* dst = s_acc + (warp * G + row) * kD + 2 * quad;
 #pragma unroll
-      for (int nb = 0; nb < 16; ++nb) *reinterpret_cast<float2*>(dst + nb * 8) = make_float2(o[nb][0] + o[nb][2], o[nb][1] + o[nb][3]);
+      for (int nb = 0; nb < 16; ++nb) {
+        const float2 v = make_float2(o[nb][0] + o[nb][2], o[nb][1] + o[nb][3]);
+        repair |= isnan(v.x) || isnan(v.y);
+        *reinterpret_cast<float2*>(dst + nb * 8) = v;
+      }
       if (quad == 0) {
         s_acc[4 * G * kD + warp * G + row] = m_run;
         s_acc[4 * G * kD + 4 * G + warp * G + row] = l_run;
       }
+    }
+    if (__any_sync(0xffffffffu, repair)) {               // (the newest token is in the cache by now, written by the warp that reads it here)
+      __syncwarp();
+      ck_repair_sums(s_acc + warp * G * kD, s_acc + 4 * G * kD + warp * G, G, fuse.qkv != nullptr ? s_q : q + (static_cast<size_t>(it.b) * nq + qh0) * kD,
+                     k_cache, v_cache, block_tables + static_cast<size_t>(it.b) * table_width, begin + warp * 16, end, it.kvh, nkv, block_size, num_blocks,
+                     scale_log2, lane);
     }
     named_barrier_sync(1, 128);
     const int d = threadIdx.x;

@@ -701,6 +701,39 @@ def test_decode_attention_keeps_weights_and_sums_in_fp32(ops, nq, nkv, n, chunk)
     ops.check_status()
 
 
+@pytest.mark.parametrize("raw", [False, True])
+@pytest.mark.parametrize("k_lens,nq,nkv", [([300, 64, 1000, 1], 16, 8), ([300, 64, 1000, 1], 32, 8), ([700, 129], 10, 2), ([500, 90], 8, 1)])
+def test_decode_attention_with_infinite_values(ops, k_lens, nq, nkv, raw):
+    """An infinite value under a positive weight makes an infinite sum, two of opposite signs, or a NaN, make a NaN; all other elements are what
+    they are without.  Among the values of cached tokens and of the newest one."""
+    S = len(k_lens)
+    q, kc, vc, b = _paged_case([1] * S, k_lens, nq, nkv, 256, seed=9)
+    b.is_prefill = False
+    qkv = _rand(S, (nq + 2 * nkv) * 128)
+    put = lambda s, tok, d, value: vc[int(b.block_tables[s, tok // 256]), :, tok % 256, d].fill_(value)
+    put(0, 5, 7, math.inf), put(0, 200, 8, -math.inf), put(0, 70, 100, math.inf), put(0, 130, 100, -math.inf), put(0, 131, 99, math.nan)
+    for s, n in enumerate(k_lens):
+        put(s, n // 2, 20, math.inf)
+        qkv[s, (nq + nkv) * 128 + 21] = math.inf                     # the newest token's, first KV head
+    if raw:
+        slots = torch.stack([b.block_tables[s, (n - 1) // 256] * 256 + (n - 1) % 256 for s, n in enumerate(k_lens)]).to(torch.int32)
+        table = ref.rope_table(4096, 128, 1e6, "cuda")
+        pos = b.context_lens - 1
+        kc1, vc1 = kc.clone(), vc.clone()
+        q1 = ops.qk_norm_rope_store(qkv, None, None, 1e-6, table, pos, slots, kc1, vc1, nq, nkv, 128)
+        want = ref.attention(q1, kc1, vc1, b.cu_seqlens_q, b.context_lens, b.block_tables, 128 ** -0.5, S)
+        got = ops.decode_attention_qkv(qkv, None, None, 1e-6, table, kc, vc, b, nq, 128 ** -0.5)
+    else:
+        want = ref.attention(q, kc, vc, b.cu_seqlens_q, b.context_lens, b.block_tables, 128 ** -0.5, S)
+        got = ops.attention(q, kc, vc, b, 128 ** -0.5)
+    got, want = got.view_as(want).float(), want.float()
+    finite = torch.isfinite(want)
+    assert (~finite).sum() > 2 * nq and torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got[got.isinf()], want[want.isinf()]) and torch.equal(got.isinf(), want.isinf())
+    _close(got[finite], want[finite], 2e-2, 2e-2)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("nq,nkv", [(16, 8), (32, 8)])
 def test_decode_attention_refuses_a_cache_that_is_not_aligned(ops, nq, nkv):
     """Every kernel copies cache rows 16 bytes at a time; a cache that begins elsewhere is an error on the host."""
