@@ -51,9 +51,9 @@ __device__ __forceinline__ int chunk_checked_len(const int* __restrict__ lens, i
   return max(len, 0);
 }
 
-// Item `item`; executed by whole warps.  Direct: of the list [chunk][sequence][KV head] with `parts` chunks for every sequence, dead ones have
+// Item `item`; executed by whole warps.  Direct: of the list [chunk][sequence][KV head] with `most` chunks for every sequence, dead ones have
 // c * chunk >= len.  Else of the list [live chunk][KV head].  False: there are not that many.
-__device__ __forceinline__ bool chunk_item(const int* __restrict__ lens, int B, int nkv, int unit, int parts, int cap, bool direct, int item,
+__device__ __forceinline__ bool chunk_item(const int* __restrict__ lens, int B, int nkv, const DecodeSplit& split, int cap, bool direct, int item,
                                            unsigned* status, ChunkItem& it) {
   const int lane = threadIdx.x & 31;
   int left = item / nkv;
@@ -61,14 +61,14 @@ __device__ __forceinline__ bool chunk_item(const int* __restrict__ lens, int B, 
   if (direct) {
     it.c = left / B;
     it.b = left - it.c * B;
-    if (it.c >= parts) return false;
+    if (it.c >= split.most) return false;
     it.len = chunk_checked_len(lens, it.b, cap, status);
-    it.chunk = decode_chunk_tokens(it.len, unit, parts);
+    it.chunk = decode_chunk_tokens(it.len, split);
     return true;
   }
   for (int b0 = 0; b0 < B; b0 += 32) {
     const int len = b0 + lane < B ? chunk_checked_len(lens, b0 + lane, cap, status) : 0;
-    const int chunk = decode_chunk_tokens(len, unit, parts), n = (len + chunk - 1) / chunk;
+    const int chunk = decode_chunk_tokens(len, split), n = (len + chunk - 1) / chunk;
     int sum = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
     const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const __nv_bfloat16* __restrict__ q,
     __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, const int* __restrict__ block_tables, const int* __restrict__ context_lens,
     __nv_bfloat16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml, int B, int nq, int nkv, int block_size,
-    int table_width, int num_blocks, int unit, int max_chunks, int parts, int direct, float scale_log2, unsigned* status, const DecodeFuse fuse) {
+    int table_width, int num_blocks, const DecodeSplit split, int max_chunks, int direct, float scale_log2, unsigned* status, const DecodeFuse fuse) {
   static_assert(G <= 8, "the heads of a group fill the first eight rows of the query tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
   uint64_t* empty_bar = full_bar + kCkStages;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int cap = min(table_width * block_size, max_chunks * unit);
+  const int cap = min(table_width * block_size, max_chunks * split.unit);
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tm_k);
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
     // ------------------------------------------------------------------ producer
     int n = 0;
     bool ok = true;
-    for (int item = blockIdx.x; ok && chunk_item(context_lens, B, nkv, unit, parts, cap, direct != 0, item, status, it); item += gridDim.x) {
+    for (int item = blockIdx.x; ok && chunk_item(context_lens, B, nkv, split, cap, direct != 0, item, status, it); item += gridDim.x) {
       if (lane == 0) {
         const int end = min(it.len, (it.c + 1) * it.chunk);
         for (int tok = it.c * it.chunk; tok < end; tok += kCkTile, ++n) {
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
   const int mat = lane >> 3, mrow = lane & 7;           // ldmatrix: this lane supplies row `mrow` of matrix `mat`
   int n = 0;
   bool ok = true;                                       // once a wait has run out none is made any more, but every barrier still is
-  for (int item = blockIdx.x; chunk_item(context_lens, B, nkv, unit, parts, cap, direct != 0, item, nullptr, it); item += gridDim.x) {
+  for (int item = blockIdx.x; chunk_item(context_lens, B, nkv, split, cap, direct != 0, item, nullptr, it); item += gridDim.x) {
     const int qh0 = it.kvh * G, begin = it.c * it.chunk, end = min(it.len, begin + it.chunk);
     if (begin >= end) continue;                         // uniform for the consumers
     // the newest token (position len - 1) is not in the cache yet: the warp that owns its row of its tile prepares it now
@@ -379,7 +379,7 @@ extern "C" int forge_make_tmap_2d(CUtensorMap* tm, const void* base, uint64_t ro
 
 template <int G>
 static int launch_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
-                         int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk, int max_chunks, int parts, float scale_log2, unsigned* status,
+                         int nq, int nkv, int block_size, int table_width, int num_blocks, const DecodeSplit& split, int max_chunks, float scale_log2, unsigned* status,
                          cudaStream_t stream, const DecodeFuse& fuse) {
   constexpr int smem = kCkStages * 2 * kCkTileBytes + decode_merge_floats(G) * 4 + G * kD * 2 + 512 + 2 * kCkStages * 8 + 1024;
   static_assert(ck_ctas_per_sm(G) * (smem + 1024) <= 228 * 1024, "CTAs per SM");
@@ -389,24 +389,24 @@ static int launch_chunks(const void* q, const void* kc, const void* vc, const in
   const uint64_t rows = static_cast<uint64_t>(num_blocks) * nkv * block_size;
   if (forge_make_tmap_2d(&tm_k, kc, rows, kD, kD, kCkTile, 2) != 0 || forge_make_tmap_2d(&tm_v, vc, rows, kD, kD, kCkTile, 2) != 0) return -2;
   // up to two waves of CTAs: one per item, dead ones included (they end at once, and no list is walked); else the live ones over one wave
-  const long long most = static_cast<long long>(B) * nkv * parts;
+  const long long most = static_cast<long long>(B) * nkv * split.most;
   const int wave = ck_ctas_per_sm(G) * device_sm_count();
   const int direct = most <= 2 * wave;
   const dim3 grid(static_cast<unsigned>(direct ? most : wave));
   return launch_kernel(kern, grid, dim3(kDecThreads), smem, stream, 0, tm_k, tm_v, static_cast<const __nv_bfloat16*>(q),
                        static_cast<__nv_bfloat16*>(const_cast<void*>(kc)), static_cast<__nv_bfloat16*>(const_cast<void*>(vc)), bt, lens,
-                       static_cast<__nv_bfloat16*>(out), part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, chunk, max_chunks, parts,
+                       static_cast<__nv_bfloat16*>(out), part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, split, max_chunks,
                        direct, scale_log2, status, fuse) == cudaSuccess ? 0 : -5;
 }
 
 // The attention kernel alone (partials of sequences of several chunks are merged by the caller); group = nq / nkv, 4..8.
 int launch_decode_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
-                         int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk, int max_chunks, int parts, float scale_log2, unsigned* status,
+                         int nq, int nkv, int block_size, int table_width, int num_blocks, const DecodeSplit& split, int max_chunks, float scale_log2, unsigned* status,
                          cudaStream_t stream, const DecodeFuse& fuse) {
 #define FORGE_CK(G)                                                                                                                          \
   case G:                                                                                                                                    \
-    return launch_chunks<G>(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, chunk, max_chunks, \
-                            parts, scale_log2, status, stream, fuse)
+    return launch_chunks<G>(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, split, max_chunks, \
+                            scale_log2, status, stream, fuse)
   switch (nq / nkv) {
     FORGE_CK(4);
     FORGE_CK(5);

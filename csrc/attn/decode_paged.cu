@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kDecThreads, decode_ctas_per_sm(G)) decode_att
     const __nv_bfloat16* __restrict__ q, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
     const int* __restrict__ block_tables, const int* __restrict__ context_lens, __nv_bfloat16* __restrict__ out,
     float* __restrict__ part_o, float* __restrict__ part_ml, int nq, int nkv, int block_size, int table_width, int num_blocks,
-    int unit, int max_chunks, int parts, float scale_log2, unsigned* status, const DecodeFuse fuse) {
+    const DecodeSplit split, int max_chunks, float scale_log2, unsigned* status, const DecodeFuse fuse) {
   constexpr int kTileBytes = TILE * kD * 2;
   static_assert(TILE >= 16 && TILE <= 64 && (TILE & (TILE - 1)) == 0, "tile");
 
@@ -56,8 +56,8 @@ __global__ void __launch_bounds__(kDecThreads, decode_ctas_per_sm(G)) decode_att
   const int qh0 = kvh * (nq / nkv) + (blockIdx.x % groups_per_kv) * G;
   const int b = blockIdx.y;
   const int c = blockIdx.z;
-  const int len = decode_checked_len(context_lens, b, min(table_width * block_size, max_chunks * unit), status);
-  const int chunk = decode_chunk_tokens(len, unit, parts);
+  const int len = decode_checked_len(context_lens, b, min(table_width * block_size, max_chunks * split.unit), status);
+  const int chunk = decode_chunk_tokens(len, split);
   const int tok_begin = c * chunk;
   if (tok_begin >= len) {                                // uniform for the CTA
     if (c == 0 && threadIdx.x < kD)                      // padding row (length 0): defined output
@@ -165,13 +165,13 @@ __device__ __forceinline__ float2 combine_load_pair(const float* __restrict__ ml
 // partial rows eight at a time: with one after another the merge of 47 chunks took 8.7 us, longer than it took to make half of them.
 __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                             const int* __restrict__ context_lens, __nv_bfloat16* __restrict__ out,
-                                                            int nq, int unit, int max_chunks, int parts, int cap) {
+                                                            int nq, const DecodeSplit split, int max_chunks, int cap) {
   __shared__ float s_w[kD], s_max[kD / 32];
   pdl_launch_dependents();
   pdl_wait();
   const int b = blockIdx.y, qh = blockIdx.x, d = threadIdx.x;
   const int len = decode_checked_len(context_lens, b, cap, nullptr);      // same clamp as the attention kernel, which reports it
-  const int chunk = decode_chunk_tokens(len, unit, parts);
+  const int chunk = decode_chunk_tokens(len, split);
   const int n = (len + chunk - 1) / chunk;
   if (n <= 1) return;
   const size_t base = (static_cast<size_t>(b) * nq + qh) * max_chunks;
@@ -232,16 +232,16 @@ __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restr
   out[(static_cast<size_t>(b) * nq + qh) * kD + d] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
 }
 
-static int launch_decode_combine(const float* part_o, const float* part_ml, const int* lens, void* out, int B, int nq, int chunk, int max_chunks, int parts, int cap,
+static int launch_decode_combine(const float* part_o, const float* part_ml, const int* lens, void* out, int B, int nq, const DecodeSplit& split, int max_chunks, int cap,
                                  cudaStream_t stream) {
-  return launch_kernel(decode_combine_kernel, dim3(nq, B), dim3(kD), 0, stream, 0, part_o, part_ml, lens, static_cast<__nv_bfloat16*>(out), nq, chunk,
-                       max_chunks, parts, cap) == cudaSuccess ? 0 : -5;
+  return launch_kernel(decode_combine_kernel, dim3(nq, B), dim3(kD), 0, stream, 0, part_o, part_ml, lens, static_cast<__nv_bfloat16*>(out), nq, split,
+                       max_chunks, cap) == cudaSuccess ? 0 : -5;
 }
 
 template <int G, int TILE>
 static int launch_decode(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o,
-                         float* part_ml, int B, int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk,
-                         int max_chunks, int parts, float scale_log2, unsigned* status, cudaStream_t stream, const DecodeFuse& fuse) {
+                         float* part_ml, int B, int nq, int nkv, int block_size, int table_width, int num_blocks, const DecodeSplit& split,
+                         int max_chunks, float scale_log2, unsigned* status, cudaStream_t stream, const DecodeFuse& fuse) {
   constexpr int kTileBytes = TILE * kD * 2;
   constexpr int merge_bytes = decode_merge_floats(G) * 4;
   constexpr int ring = kDecStages * 2 * kTileBytes;
@@ -249,24 +249,25 @@ static int launch_decode(const void* q, const void* kc, const void* vc, const in
   auto kern = decode_attn_kernel<G, TILE>;
   FORGE_ENSURE_DYN_SMEM(kern, smem);
   const int groups_per_kv = (nq / nkv) / G;
-  dim3 grid(nkv * groups_per_kv, B, parts);
+  dim3 grid(nkv * groups_per_kv, B, split.most);
   if (launch_kernel(kern, grid, dim3(kDecThreads), smem, stream, 0, static_cast<const __nv_bfloat16*>(q),
                     static_cast<__nv_bfloat16*>(const_cast<void*>(kc)), static_cast<__nv_bfloat16*>(const_cast<void*>(vc)), bt, lens,
-                    static_cast<__nv_bfloat16*>(out), part_o, part_ml, nq, nkv, block_size, table_width, num_blocks, chunk,
-                    max_chunks, parts, scale_log2, status, fuse) != cudaSuccess)
+                    static_cast<__nv_bfloat16*>(out), part_o, part_ml, nq, nkv, block_size, table_width, num_blocks, split,
+                    max_chunks, scale_log2, status, fuse) != cudaSuccess)
     return -5;
   if (max_chunks > 1)
-    return launch_decode_combine(part_o, part_ml, lens, out, B, nq, chunk, max_chunks, parts, std::min(table_width * block_size, max_chunks * chunk), stream);
+    return launch_decode_combine(part_o, part_ml, lens, out, B, nq, split, max_chunks, std::min(table_width * block_size, max_chunks * split.unit), stream);
   return 0;
 }
 
 int launch_decode_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
-                         int nq, int nkv, int block_size, int table_width, int num_blocks, int chunk, int max_chunks, int parts, float scale_log2, unsigned* status,
+                         int nq, int nkv, int block_size, int table_width, int num_blocks, const DecodeSplit& split, int max_chunks, float scale_log2, unsigned* status,
                          cudaStream_t stream, const DecodeFuse& fuse);
 
 // q [B, nq, 128] bf16; caches [num_blocks, nkv, block_size, 128] bf16; block_tables [B, table_width]; out [B, nq * 128].
 // part_o: fp32 [B, nq, max_chunks, 128], part_ml: fp32 [B, nq, max_chunks, 2] (may be null when max_chunks == 1).
-// chunk: tokens per grid.z slice, a multiple of min(block_size, 64); max_chunks * chunk must cover the longest context.
+// chunk: tokens of the smallest chunk, a multiple of min(block_size, 64), of which longer ones are multiples; max_chunks * chunk must cover the
+// longest context.
 static int decode_chunked_impl(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out,
                                float* part_o, float* part_ml, int B, int nq, int nkv, int head_dim, int block_size,
                                int table_width, int num_blocks, int chunk, int max_chunks, float scale, unsigned* status,
@@ -280,20 +281,25 @@ static int decode_chunked_impl(const void* q, const void* kc, const void* vc, co
   const int group = nq / nkv;
   const int G = decode_group_slice(group);
   const float sl2 = scale * 1.4426950408889634f;
-  // Very few sequences: at most 24 chunks each, more of them cost the merge more than they save (3001 tokens of 32 / 8 heads: 47 chunks 15.5 us, 24: 13.3).
-  const int parts = B * nkv < 32 ? std::min(max_chunks, 24) : max_chunks;
+  // Few sequences: at most kFewChunks chunks each, or as many as give every SM one.  More of them cost the merge more than they save, and with 8 KV
+  // heads 24 are near the best at any length; with fewer heads a long context needs more to occupy the GPU (decode_chunk_tokens says how many).
+  // Measured, us with chunks of 64 tokens / 24 chunks / this rule, one sequence of 3001, 8000, 32000 tokens: 32 / 8 heads 13.6, 29.6, 98 / 11.8, 16.9, 34.4
+  // (the same); 16 / 8: 13.4, 26.1, 100 / 9.7, 13.9, 30.4 (the same); 4 / 1 heads: 9.2, 15.4, 45.8 / 8.8, 11.8, 25.4 / 8.8, 10.9, 17.7;
+  // 2 / 1: 7.6, 13.1, 42.2 / 6.8, 10.0, 21.7 / 6.8, 9.5, 15.6; 4 sequences of 4 / 1 heads: 11.7, 22.4, 67.9 / 10.4, 14.4, 27.2 / 10.4, 13.9, 25.
+  const int few = B * nkv < 32;
+  const DecodeSplit split = {chunk, few ? std::min(max_chunks, std::max(kFewChunks, device_sm_count() / (B * nkv))) : max_chunks, few};
   // Groups of 4 to 8 heads, cache blocks of 64 tokens and more: on the tensor cores (decode_chunks.cu).  With two heads per
   // KV head the CUDA cores keep up with the stream and their kernel starts faster (2 sequences 12.0 us against 13.8, 40: 44 against 53); with four
   // they do not (13 sequences: 31.7 against 22.4).
   if (tile == 64 && group >= 4 && group <= 8) {
-    const int rc = launch_decode_chunks(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, chunk, max_chunks, parts, sl2,
+    const int rc = launch_decode_chunks(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, split, max_chunks, sl2,
                                         status, stream, fuse);
     if (rc != 0 || max_chunks <= 1) return rc;
-    return launch_decode_combine(part_o, part_ml, lens, out, B, nq, chunk, max_chunks, parts, std::min(table_width * block_size, max_chunks * chunk), stream);
+    return launch_decode_combine(part_o, part_ml, lens, out, B, nq, split, max_chunks, std::min(table_width * block_size, max_chunks * split.unit), stream);
   }
 #define FORGE_DEC(GG, TT)                                                                                                   \
   return launch_decode<GG, TT>(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, \
-                               chunk, max_chunks, parts, sl2, status, stream, fuse)
+                               split, max_chunks, sl2, status, stream, fuse)
   if (tile == 64) {
     if (G == 5) FORGE_DEC(5, 64);
     if (G == 4) FORGE_DEC(4, 64);

@@ -618,6 +618,21 @@ def test_decode_attention_from_raw_qkv(ops, k_lens, nq, nkv, bs, mode, monkeypat
     ops.check_status()
 
 
+@pytest.mark.parametrize("nq,nkv", [(8, 8), (16, 8), (24, 8), (32, 8), (40, 8), (64, 8), (2, 1), (5, 1)])
+def test_decode_attention_with_chunks_longer_than_asked_for(ops, nq, nkv, monkeypatch):
+    """One sequence of 2000 tokens under a table for more, from ready queries and from the raw projection."""
+    test_decode_attention_from_raw_qkv(ops, [2000], nq, nkv, 256, "chunked", monkeypatch)
+    test_decode_attention(ops, [2000], nq, nkv, 256, "chunked", monkeypatch)
+
+
+@pytest.mark.parametrize("nq", [32, 64])
+def test_decode_attention_from_raw_qkv_over_a_list_of_chunks(ops, nq, monkeypatch):
+    """More possible chunks than two waves of CTAs: each walks the list of live ones, several in a row, through one ring."""
+    k_lens = [(1 + 977 * i) % 4000 for i in range(32)]
+    k_lens[5] = k_lens[31] = 0
+    test_decode_attention_from_raw_qkv(ops, k_lens, nq, 8, 256, "chunked", monkeypatch)
+
+
 @pytest.mark.parametrize("k_lens,nq,nkv", [([300, 1000, 70, 2], 32, 8), ([129, 640, 33, 2011], 40, 8), ([50, 400, 900], 8, 2)])
 def test_decode_attention_cuda_core_variant_for_groups_of_4_and_5(ops, k_lens, nq, nkv, monkeypatch):
     """The flat kernel runs groups of 4..8 q heads per KV head on the tensor cores by default (covered by the tests above); the
@@ -638,12 +653,14 @@ def test_decode_attention_cuda_core_variant_for_groups_of_4_and_5(ops, k_lens, n
 
 @pytest.mark.parametrize("k_lens,nq,nkv,bs,chunk,max_chunks", [
     ([1, 63, 64, 65, 0, 128, 129, 700], 32, 8, 256, 64, 16),           # edges of tiles and chunks, a padding row, every sequence cut
-    ([2000, 5], 8, 2, 64, 64, 32),                                     # at most 24 chunks: longer ones than asked for
+    ([2000, 5], 8, 2, 64, 64, 32),                                     # few sequences: fewer and longer chunks than asked for
+    ([9000], 4, 1, 256, 64, 141), ([9000], 2, 1, 256, 64, 141), ([20000, 3000], 5, 1, 512, 64, 313),      # more than 24 of them
+    ([9000, 1, 700, 3000], 32, 8, 256, 64, 141), ([9000, 1, 700, 3000], 16, 8, 256, 64, 141),             # more than 128 to merge
     ([0, 640, 641, 1], 10, 2, 128, 128, 6), ([300, 511], 12, 2, 256, 64, 8), ([300, 511], 7, 1, 256, 256, 2), ([900] * 3, 16, 2, 512, 1024, 1),
     ([17 * i % 900 for i in range(70)], 32, 8, 256, 64, 15),           # more items than two waves: walked as a list, three ballots of sequences
 ])
 def test_decode_attention_chunks_on_tensor_cores(ops, k_lens, nq, nkv, bs, chunk, max_chunks):
-    """Groups of 4 to 8 heads; the weights keep 16 bits, so what is left is the rounding of the bf16 result (2^-9 of values of unit size)."""
+    """Groups of 4 to 8 heads (and one of 2); weights and sums are fp32, so what is left is the rounding of the bf16 result (2^-9 of values of unit size)."""
     q, kc, vc, b = _paged_case([1] * len(k_lens), k_lens, nq, nkv, bs, seed=4)
     want = ref.attention(q, kc, vc, b.cu_seqlens_q, b.context_lens, b.block_tables, 128 ** -0.5, b.num_seqs)
     B = len(k_lens)
