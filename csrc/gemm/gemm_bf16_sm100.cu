@@ -1969,10 +1969,10 @@ extern "C" int forge_gemm_bf16_qkv(const void* x, int ldx, const void* w, int ld
   const int n_out = (nq + 2 * nkv) * 128;
   TpPush none = {};
   // Prompts: the CTA-pair kernel, like the plain projection.  A tile's 64 KB of cos / sin values and the longer epilogue hide behind
-  // the products; what goes is a pass over q, k and v (written, read and written again).
-  // With the pass as a kernel of its own / in here: 3777 tokens, K 4096, 32 + 16 heads: 180 / 149 us; 2048: 111 / 99; 8192, K 2560: 224 / 206.
-  // With K 1024 the products of a tile are shorter than its epilogue (15717 tokens, 16 + 16 heads: 162 / 165; 2000: 32 / 36): callers
-  // keep the two kernels there.
+  // the products of the pair's next tile; what goes is a pass over q, k and v (written, read and written again).
+  // With the pass as a kernel of its own / in here: 3777 tokens, K 4096, 32 + 16 heads: 162 / 146 us; 2048: 102 / 90; 8192, K 2560: 220 / 196.
+  // Where a pair has one tile only, or products too short to hide the epilogue (K 1024: 15700 tokens 162 / 171, 2000: 27 / 32), callers keep
+  // the two kernels.
   if (M > 256) return launch_pair<kEpiQkv>(x, ldx, w, n_out, ldw, nullptr, 0, M, n_out, K, status, stream, none, fuse, 0, 0, 0, qk);
   return launch_tokens<128, kEpiQkv>(x, ldx, w, n_out, ldw, nullptr, 0, M, n_out, K, status, stream, none, fuse, GemmSample{}, 0, 0, 0, qk);
 }

@@ -385,20 +385,32 @@ def test_qkv_gemm_of_prompts_with_norm_rope_and_cache_store_in_its_epilogue(ops,
     test_qkv_gemm_with_norm_rope_and_cache_store_in_its_epilogue(ops, T, K, nq, nkv, bs, folded)
 
 
-@pytest.mark.parametrize("T,K,nq,nkv", [(300, 2048, 16, 8), (1500, 4096, 5, 1)])
-def test_qkv_gemm_of_prompts_gives_the_bits_of_the_two_kernels(ops, T, K, nq, nkv):
+@pytest.mark.parametrize("folded", [True, False])
+@pytest.mark.parametrize("T,K,nq,nkv", [(300, 2048, 16, 8), (1500, 4096, 5, 1), (2000, 4096, 16, 4), (700, 2560, 8, 2)])
+def test_qkv_gemm_of_prompts_gives_the_bits_of_the_two_kernels(ops, T, K, nq, nkv, folded):
+    """With the input norm folded in (one GPU) and without it (ranks of several, which hold a part of the heads)."""
     torch.manual_seed(T)
     x, w = _rand(T, K), _rand((nq + 2 * nkv) * 128, K, scale=0.05)
     qw, kw = _rand(128, scale=0.2) + 1, _rand(128, scale=0.2) + 1
-    ssq = (x.float() ** 2).view(T, K // 128, -1).sum(-1).contiguous()
+    ssq = (x.float() ** 2).view(T, K // 128, -1).sum(-1).contiguous() if folded else None
     table = ref.rope_table(4096, 128, 1e6, "cuda")
     pos = torch.randint(0, 4096, (T,), dtype=torch.int32, device="cuda")
     slots = torch.randperm(2048, device="cuda")[:T].to(torch.int32)
     caches = [torch.zeros(8, nkv, 256, 128, dtype=BF, device="cuda") for _ in range(4)]
     got = ops.linear_qkv_rope_store(x, w, ssq, 1e-6, qw, kw, 1e-6, table, pos, slots, caches[0], caches[1], nq, nkv)
-    want = ops.qk_norm_rope_store(ops.linear_scaled(x, w, ssq, 1e-6), qw, kw, 1e-6, table, pos, slots, caches[2], caches[3], nq, nkv, 128)
+    proj = ops.linear_scaled(x, w, ssq, 1e-6) if folded else ops.linear(x, w)
+    want = ops.qk_norm_rope_store(proj, qw, kw, 1e-6, table, pos, slots, caches[2], caches[3], nq, nkv, 128)
     assert torch.equal(got.view(-1), want.view(-1)) and torch.equal(caches[0], caches[2]) and torch.equal(caches[1], caches[3])
     ops.check_status()
+
+
+def test_qkv_gemm_route_of_prompts(ops):
+    """One kernel where pairs have several tiles each (74 pairs; hidden sizes from 4096) or many (2560); two kernels else, as for fp8 weights."""
+    weight = lambda heads, hidden: torch.empty(heads * 128, hidden, dtype=BF, device="meta")
+    route = lambda rows, heads, hidden: ops.qkv_rope_store_in_gemm(rows, 128, weight(heads, hidden), True)
+    assert route(3777, 48, 4096) and route(1024, 48, 4096) and route(2048, 24, 4096) and route(3777, 48, 2560) and route(8192, 6, 4096)
+    assert not (route(300, 48, 4096) or route(768, 48, 4096) or route(1024, 24, 4096) or route(3777, 6, 4096) or route(1500, 48, 2560))
+    assert not (route(200, 48, 4096) or route(16000, 32, 2048) or route(16000, 32, 1024) or ops.qkv_rope_store_in_gemm(3777, 64, weight(48, 4096), True))
 
 
 def test_embedding_sum_of_squares(ops):

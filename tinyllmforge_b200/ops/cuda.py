@@ -263,20 +263,28 @@ class CudaOps(MixerOps, HybridOps):
         return q
 
     def qkv_rope_store_in_gemm(self, rows: int, head_dim: int, weight, prefill: bool = False) -> bool:
-        """Whether the epilogue of the qkv projection does the per-head norm, the rotation and the cache write: steps of more than 256
-        rows of a hidden size from 2048 (CTA-pair kernel, two heads per tile; measured 180 -> 149 us with 3777 tokens of size 4096,
-        224 -> 206 with 8192 of 2560, but 162 -> 165 with 15717 of 1024, whose products are too short to hide the epilogue), and, if asked
-        for, decode steps of 33..256 (tiles of 128 features = one head); with head_dim 128 and a bf16 qkv weight."""
+        """Whether the epilogue of the qkv projection does the per-head norm, the rotation and the cache write, with head_dim 128 and a
+        bf16 weight: steps of more than 256 rows (CTA-pair kernel, two heads per 256 x 256 tile) where enough of the epilogue hides behind the
+        products of another tile, and, if asked for, decode steps of 33..256 (tiles of 128 features = one head).
+
+        Measured, two kernels / one, us: hidden size 4096, 32 + 16 heads (24 tiles to 256 rows): 512 rows 35.9 / 34.3, 1024: 57 / 53, 2048: 102 / 90,
+        3777: 162 / 146; a rank's 16 + 8 heads: 512 rows 30.0 / 32.7, 1536 (72 tiles) 36 / 39, 2048 (96) 58 / 53; 4 + 2 heads: 3777 (45) 33.6 / 33.7,
+        8192 (96) 57 / 53.  A pair with one tile has nothing to hide its epilogue behind, so from 4096 on it takes more tiles than pairs.  Products of
+        2560 are shorter than the epilogue of their tile: 1300 rows (144 tiles) 45 / 47, 3000 (288) 89 / 90, 3777 (360) 116 / 99; more than four waves.
+        With 2048 (1024) some row counts gain and others lose up to 10 % (20 %): 3000 rows of 16 + 16 heads 51 / 56, 8192 121 / 114."""
         if head_dim != 128 or isinstance(weight, Fp8BlockWeight) or weight.dtype != torch.bfloat16:
             return False
         if rows > 256:
-            return weight.shape[1] >= 2048
+            features, hidden = weight.shape
+            tiles, pairs = -(-rows // 256) * -(-features // 256), self.num_sms // 2
+            return hidden >= 4096 and tiles > pairs or hidden >= 2560 and tiles > 4 * pairs
         return self.qkv_epilogue and self.qkv_epilogue_min_rows <= rows and not prefill
 
     def linear_qkv_rope_store(self, x, w, ssq_row, in_eps, q_weight, k_weight, eps, table, positions, slot_mapping, k_cache, v_cache,
                               num_heads, num_kv_heads, do_rope=True):
         """qkv projection (optionally with the folded input norm, see ``linear_scaled``) + q/k-norm + RoPE + KV store in
-        one kernel; returns q [T, heads, 128].  Replaces linear + qk_norm_rope_store for decode steps."""
+        one kernel; returns q [T, heads, 128].  Replaces linear + qk_norm_rope_store where ``qkv_rope_store_in_gemm`` says so; from
+        257 rows on the bits are those of the two."""
         T = x.shape[0]
         q = torch.empty(T, num_heads, 128, dtype=x.dtype, device=x.device)
         self.C.gemm_qkv_rope_store(x, w, ssq_row, in_eps, q_weight, k_weight, eps, table, positions, slot_mapping, q, k_cache, v_cache,
