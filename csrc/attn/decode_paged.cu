@@ -267,11 +267,12 @@ int launch_decode_chunks(const void* q, const void* kc, const void* vc, const in
 // q [B, nq, 128] bf16; caches [num_blocks, nkv, block_size, 128] bf16; block_tables [B, table_width]; out [B, nq * 128].
 // part_o: fp32 [B, nq, max_chunks, 128], part_ml: fp32 [B, nq, max_chunks, 2] (may be null when max_chunks == 1).
 // chunk: tokens of the smallest chunk, a multiple of min(block_size, 64), of which longer ones are multiples; max_chunks * chunk must cover the
-// longest context.
+// longest context.  keep_order: chunks of exactly that size, on the CUDA cores whatever the group: every head's sums in one order, which neither the
+// number of sequences nor the choice of a kernel changes.  For callers to whom the last bit of the result matters more than its time.
 static int decode_chunked_impl(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out,
                                float* part_o, float* part_ml, int B, int nq, int nkv, int head_dim, int block_size,
                                int table_width, int num_blocks, int chunk, int max_chunks, float scale, unsigned* status,
-                               cudaStream_t stream, const DecodeFuse& fuse) {
+                               cudaStream_t stream, const DecodeFuse& fuse, int keep_order) {
   if (B <= 0) return 0;
   if (head_dim != kD || nq % nkv != 0 || block_size < 16 || (block_size & (block_size - 1))) return -1;
   const int tile = block_size < 64 ? block_size : 64;
@@ -286,12 +287,12 @@ static int decode_chunked_impl(const void* q, const void* kc, const void* vc, co
   // Measured, us with chunks of 64 tokens / 24 chunks / this rule, one sequence of 3001, 8000, 32000 tokens: 32 / 8 heads 13.6, 29.6, 98 / 11.8, 16.9, 34.4
   // (the same); 16 / 8: 13.4, 26.1, 100 / 9.7, 13.9, 30.4 (the same); 4 / 1 heads: 9.2, 15.4, 45.8 / 8.8, 11.8, 25.4 / 8.8, 10.9, 17.7;
   // 2 / 1: 7.6, 13.1, 42.2 / 6.8, 10.0, 21.7 / 6.8, 9.5, 15.6; 4 sequences of 4 / 1 heads: 11.7, 22.4, 67.9 / 10.4, 14.4, 27.2 / 10.4, 13.9, 25.
-  const int few = B * nkv < 32;
+  const int few = B * nkv < 32 && keep_order == 0;
   const DecodeSplit split = {chunk, few ? std::min(max_chunks, std::max(kFewChunks, device_sm_count() / (B * nkv))) : max_chunks, few};
   // Groups of 4 to 8 heads, cache blocks of 64 tokens and more: on the tensor cores (decode_chunks.cu).  With two heads per
   // KV head the CUDA cores keep up with the stream and their kernel starts faster (2 sequences 12.0 us against 13.8, 40: 44 against 53); with four
   // they do not (13 sequences: 31.7 against 22.4).
-  if (tile == 64 && group >= 4 && group <= 8) {
+  if (tile == 64 && group >= 4 && group <= 8 && keep_order == 0) {
     const int rc = launch_decode_chunks(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, split, max_chunks, sl2,
                                         status, stream, fuse);
     if (rc != 0 || max_chunks <= 1) return rc;
@@ -325,10 +326,10 @@ static int decode_chunked_impl(const void* q, const void* kc, const void* vc, co
 extern "C" int forge_decode_attention(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out,
                                       float* part_o, float* part_ml, int B, int nq, int nkv, int head_dim, int block_size,
                                       int table_width, int num_blocks, int chunk, int max_chunks, float scale, unsigned* status,
-                                      cudaStream_t stream) {
+                                      cudaStream_t stream, int keep_order) {
   const DecodeFuse none = {};
   return decode_chunked_impl(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, head_dim, block_size, table_width, num_blocks,
-                             chunk, max_chunks, scale, status, stream, none);
+                             chunk, max_chunks, scale, status, stream, none, keep_order);
 }
 
 
@@ -1002,7 +1003,7 @@ extern "C" int forge_decode_attention_qkv(const void* qkv, int ld_qkv, const voi
                                           int rope_rows, void* kc, void* vc, const int* bt, const int* lens, void* out, float* scratch,
                                           int num_ctas, float* part_o, float* part_ml, int chunk, int max_chunks, int B, int nq, int nkv,
                                           int head_dim, int block_size, int table_width, int num_blocks, float scale, unsigned* status,
-                                          cudaStream_t stream) {
+                                          cudaStream_t stream, int keep_order) {
   if (qkv == nullptr || (ld_qkv & 7) || (reinterpret_cast<uintptr_t>(qkv) & 15)) return -1;
   DecodeFuse fuse;
   fuse.qkv = static_cast<const __nv_bfloat16*>(qkv);
@@ -1016,7 +1017,7 @@ extern "C" int forge_decode_attention_qkv(const void* qkv, int ld_qkv, const voi
     return decode_flat_impl(nullptr, kc, vc, bt, lens, out, scratch, num_ctas, B, nq, nkv, head_dim, block_size, table_width, num_blocks,
                             scale, status, stream, fuse);
   return decode_chunked_impl(nullptr, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, head_dim, block_size, table_width, num_blocks,
-                             chunk, max_chunks, scale, status, stream, fuse);
+                             chunk, max_chunks, scale, status, stream, fuse, keep_order);
 }
 
 
@@ -1068,7 +1069,7 @@ enum ForgeNoAllocError {
 extern "C" const char* forge_decode_attention_noalloc_strerror(int code) {
   switch (code) {
     case FORGE_NOALLOC_OK: return "ok";
-    case FORGE_NOALLOC_BAD_ARGUMENT: return "bad argument: head_dim must be 128, block_size a power of two >= 16, chunk a multiple of min(block_size, 64)";
+    case FORGE_NOALLOC_BAD_ARGUMENT: return "bad argument: head_dim must be 128, block_size a power of two >= 16, chunk a multiple of min(block_size, 64), caches aligned to 16 bytes";
     case FORGE_NOALLOC_TOO_LARGE: return "B * nq * max_chunks * 130 floats exceed the built-in 16 MiB scratch array; use forge_decode_attention with caller-provided scratch";
     case FORGE_NOALLOC_SYMBOL_LOOKUP_FAILED: return "cudaGetSymbolAddress failed for the built-in scratch array on the current device";
     case FORGE_NOALLOC_LAUNCH_FAILED: return "kernel launch failed";
@@ -1097,7 +1098,7 @@ extern "C" int forge_decode_attention_noalloc(const void* q, const void* kc, con
   float* part_o = g_noalloc_scratch_dev[dev];
   float* part_ml = part_o + slots * kD;
   const int rc = forge_decode_attention(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, head_dim, block_size, table_width,
-                                        num_blocks, chunk, max_chunks, scale, status, stream);
+                                        num_blocks, chunk, max_chunks, scale, status, stream, 0);
   if (rc == -1) return FORGE_NOALLOC_BAD_ARGUMENT;
   return rc == 0 ? FORGE_NOALLOC_OK : FORGE_NOALLOC_LAUNCH_FAILED;
 }

@@ -73,7 +73,7 @@ int forge_sample(const void* logits, int fp32, int ld, int rows, int vocab, int 
 int forge_sample_merge_ranks(const float* vals, const int* ids, int ranks, int rows, int* out_i, cudaStream_t stream);
 int forge_decode_attention(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out,
                            float* part_o, float* part_ml, int B, int nq, int nkv, int head_dim, int block_size, int table_width,
-                           int num_blocks, int chunk, int max_chunks, float scale, unsigned* status, cudaStream_t stream);
+                           int num_blocks, int chunk, int max_chunks, float scale, unsigned* status, cudaStream_t stream, int keep_order);
 size_t forge_decode_attention_flat_scratch_floats(int num_ctas, int B, int nq, int nkv);
 int forge_decode_attention_flat_ctas_per_sm(int nq, int nkv, int block_size, int from_raw_qkv);
 void forge_decode_attention_set_tc_min_group(int g);
@@ -84,7 +84,7 @@ int forge_decode_attention_qkv(const void* qkv, int ld_qkv, const void* q_w, con
                                int rope_rows, void* kc, void* vc, const int* bt, const int* lens, void* out, float* scratch,
                                int num_ctas, float* part_o, float* part_ml, int chunk, int max_chunks, int B, int nq, int nkv,
                                int head_dim, int block_size, int table_width, int num_blocks, float scale, unsigned* status,
-                               cudaStream_t stream);
+                               cudaStream_t stream, int keep_order);
 int forge_prefill_attention(const void* q, const void* kc, const void* vc, const int* cu_q, const int* lens, const int* bt,
                             void* out, int T, int num_seqs, int max_q, int nq, int nkv, int head_dim, int block_size,
                             int table_width, int num_blocks, float scale, unsigned* status, cudaStream_t stream);
@@ -360,7 +360,7 @@ void sample_merge_ranks(const Tensor& vals, const Tensor& ids, Tensor& out_i) {
 
 void decode_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& block_tables,
                       const Tensor& context_lens, Tensor& out, const c10::optional<Tensor>& part_o,
-                      const c10::optional<Tensor>& part_ml, int64_t chunk, int64_t max_chunks, double scale, const Tensor& status) {
+                      const c10::optional<Tensor>& part_ml, int64_t chunk, int64_t max_chunks, double scale, const Tensor& status, bool keep_order) {
   CHECK_CUDA_CONTIG(q); CHECK_BF16(q); CHECK_CUDA_CONTIG(k_cache); CHECK_BF16(k_cache); CHECK_CUDA_CONTIG(v_cache); CHECK_BF16(v_cache);
   CHECK_CUDA_CONTIG(block_tables); CHECK_I32(block_tables); CHECK_CUDA_CONTIG(context_lens); CHECK_I32(context_lens);
   CHECK_CUDA_CONTIG(out); CHECK_BF16(out);
@@ -383,7 +383,7 @@ void decode_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
                                context_lens.data_ptr<int>(), out.data_ptr(), po, pml, static_cast<int>(B), static_cast<int>(nq),
                                static_cast<int>(nkv), static_cast<int>(D), static_cast<int>(bs), static_cast<int>(block_tables.size(1)),
                                static_cast<int>(k_cache.size(0)), static_cast<int>(chunk), static_cast<int>(max_chunks),
-                               static_cast<float>(scale), status_ptr(status), stream_of(q)),
+                               static_cast<float>(scale), status_ptr(status), stream_of(q), keep_order ? 1 : 0),
         "forge_decode_attention");
 }
 
@@ -427,7 +427,7 @@ void decode_attention_qkv(const Tensor& qkv, const c10::optional<Tensor>& qw, co
                           const c10::optional<Tensor>& rope, Tensor& k_cache, Tensor& v_cache, const Tensor& block_tables,
                           const Tensor& context_lens, Tensor& out, const c10::optional<Tensor>& scratch, int64_t num_ctas,
                           const c10::optional<Tensor>& part_o, const c10::optional<Tensor>& part_ml, int64_t chunk, int64_t max_chunks,
-                          int64_t nq, double scale, const Tensor& status) {
+                          int64_t nq, double scale, const Tensor& status, bool keep_order) {
   CHECK_BF16(qkv); CHECK_CUDA_CONTIG(k_cache); CHECK_BF16(k_cache); CHECK_CUDA_CONTIG(v_cache); CHECK_BF16(v_cache);
   CHECK_CUDA_CONTIG(block_tables); CHECK_I32(block_tables); CHECK_CUDA_CONTIG(context_lens); CHECK_I32(context_lens);
   CHECK_CUDA_CONTIG(out); CHECK_BF16(out);
@@ -461,7 +461,7 @@ void decode_attention_qkv(const Tensor& qkv, const c10::optional<Tensor>& qw, co
                                    out.data_ptr(), sp, static_cast<int>(num_ctas), po, pml, static_cast<int>(chunk),
                                    static_cast<int>(max_chunks), static_cast<int>(B), static_cast<int>(nq), static_cast<int>(nkv),
                                    static_cast<int>(D), static_cast<int>(bs), static_cast<int>(block_tables.size(1)),
-                                   static_cast<int>(k_cache.size(0)), static_cast<float>(scale), status_ptr(status), stream_of(qkv)),
+                                   static_cast<int>(k_cache.size(0)), static_cast<float>(scale), status_ptr(status), stream_of(qkv), keep_order ? 1 : 0),
         "forge_decode_attention_qkv");
 }
 
@@ -712,9 +712,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sample_nsplit", &sample_nsplit);
   m.def("sample", &sample);
   m.def("sample_merge_ranks", &sample_merge_ranks);
-  m.def("decode_attention", &decode_attention);
+  m.def("decode_attention", &decode_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_tables"), py::arg("context_lens"),
+        py::arg("out"), py::arg("part_o"), py::arg("part_ml"), py::arg("chunk"), py::arg("max_chunks"), py::arg("scale"), py::arg("status"),
+        py::arg("keep_order") = false);
   m.def("decode_attention_flat", &decode_attention_flat);
-  m.def("decode_attention_qkv", &decode_attention_qkv);
+  m.def("decode_attention_qkv", &decode_attention_qkv, py::arg("qkv"), py::arg("q_weight"), py::arg("k_weight"), py::arg("eps"), py::arg("rope"),
+        py::arg("k_cache"), py::arg("v_cache"), py::arg("block_tables"), py::arg("context_lens"), py::arg("out"), py::arg("scratch"),
+        py::arg("num_ctas"), py::arg("part_o"), py::arg("part_ml"), py::arg("chunk"), py::arg("max_chunks"), py::arg("num_heads"), py::arg("scale"),
+        py::arg("status"), py::arg("keep_order") = false);
   m.def("decode_attention_flat_scratch_floats", &decode_attention_flat_scratch_floats);
   m.def("decode_attention_flat_ctas_per_sm", &decode_attention_flat_ctas_per_sm);
   m.def("gemm_set_streamk_workspace", [](torch::Tensor ws, torch::Tensor counters, int64_t ctas) {

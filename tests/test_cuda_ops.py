@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from tinyllmforge_b200.ops import ref
+from tinyllmforge_b200.ops.cuda import decode_chunking
 
 pytestmark = pytest.mark.gpu
 
@@ -760,6 +761,41 @@ def test_decode_attention_with_infinite_values(ops, k_lens, nq, nkv, raw):
     assert (~finite).sum() > 2 * nq and torch.equal(got.isnan(), want.isnan())
     assert torch.equal(got[got.isinf()], want[want.isinf()]) and torch.equal(got.isinf(), want.isinf())
     _close(got[finite], want[finite], 2e-2, 2e-2)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("raw", [False, True])
+@pytest.mark.parametrize("k_lens,nkv", [([2000], 8), ([200 + 131 * i for i in range(13)], 8), ([3000, 70], 1)])
+def test_decode_attention_that_keeps_its_order(ops, k_lens, nkv, raw, monkeypatch):
+    """Models with fp8 weights: four heads per KV head bit for bit as two pairs of them, which always run on the CUDA cores, and in chunks of
+    exactly the size that batch and KV heads ask for, whatever the group."""
+    B = len(k_lens)
+    q, kc, vc, b = _paged_case([1] * B, k_lens, 4 * nkv, nkv, 256, seed=12)
+    b.is_prefill = False
+    qkv = _rand(B, 6 * nkv * 128)
+    monkeypatch.setattr(ops, "decode_attention_mode", "chunked")
+    monkeypatch.setattr(ops, "decode_keep_order", True)
+    def run(heads):
+        if not raw:
+            return ops.attention(q.view(B, nkv, 4, 128)[:, :, heads].reshape(B, -1, 128).contiguous(), kc, vc, b, 128 ** -0.5)
+        part = qkv.view(B, 6 * nkv, 128)
+        part = torch.cat([part[:, :4 * nkv].view(B, nkv, 4, 128)[:, :, heads].reshape(B, -1, 128), part[:, 4 * nkv:]], 1).reshape(B, -1).contiguous()
+        return ops.decode_attention_qkv(part, None, None, 1e-6, None, kc, vc, b, len(heads) * nkv, 128 ** -0.5, do_rope=False)
+    whole = run([0, 1, 2, 3]).view(B, nkv, 4, 128)
+    for pair in ([0, 1], [2, 3]):
+        assert torch.equal(run(pair).view(B, nkv, 2, 128), whole[:, :, pair])
+    chunk = decode_chunking(B, nkv, 256, b.table_width * 256)[0]
+    assert chunk == (64 if B * nkv < 16 else 256)
+    chunks = -(-max(k_lens) // chunk)
+    part_o, part_ml = torch.empty(B * 4 * nkv * chunks * 128, device="cuda"), torch.full((B * 4 * nkv * chunks * 2,), float("nan"), device="cuda")
+    out = torch.empty(B, 4 * nkv * 128, dtype=BF, device="cuda")
+    ops.C.decode_attention(q, kc, vc, b.block_tables, b.context_lens, out, part_o, part_ml, chunk, chunks, 128 ** -0.5, ops.status, True)
+    for s, n in enumerate(k_lens):
+        live = -(-n // chunk)
+        if live > 1:
+            assert not torch.isnan(part_ml.view(B, 4 * nkv, chunks, 2)[s, :, :live]).any() and torch.isnan(part_ml.view(B, 4 * nkv, chunks, 2)[s, :, live:]).all()
+    if not raw:
+        assert torch.equal(out, whole.reshape(B, -1))
     ops.check_status()
 
 

@@ -43,8 +43,10 @@ def decode_chunking(batch: int, num_kv_heads: int, block_size: int, max_len: int
 
     Small batches split the context finely so that every SM gets work; large batches keep chunks long so
     that the partial-merge traffic stays negligible.  Depends only on shapes known at graph-capture time.
+    The kernel may make chunks a multiple of this long (few sequences); the number of chunks is what scratch is sized for.
     Groups of 4 to 8 query heads run on the tensor cores with a fixed cost per chunk, which longer chunks share: measured with 32 / 8
-    heads and 200..2000 tokens, chunks of 128 / 256 / 512: 4 sequences 14.5 / 14.8 / 16.7 us, 8: 22.9 / 17.2 / 19.3, 13: 35.2 / 27.6 / 22.4, 24: 63 / 47 / 40."""
+    heads and 200..2000 tokens, chunks of 128 / 256 / 512: 4 sequences 14.5 / 14.8 / 16.7 us, 8: 22.9 / 17.2 / 19.3, 13: 35.2 / 27.6 / 22.4, 24: 63 / 47 / 40;
+    with 8 / 1 heads these sizes give 10.4 us for 8 sequences, 11.5 for 13, 9.9 for 24, 13.1 for 40 (CUDA cores and their sizes: 14.6, 21.3, 16.4, 18.3)."""
     tile = min(block_size, 64)
     ctas = batch * num_kv_heads
     if 4 <= group <= 8 and tile == 64:
@@ -100,6 +102,11 @@ class CudaOps(MixerOps, HybridOps):
         # 0.69-0.75 of copy bandwidth at 64-96 sequences, equal from 128, a few us slower below 16).
         # Scratch of the flat kernel, sized for any head grouping (~1.2 MB).
         self.decode_attention_mode = os.environ.get("FORGE_DECODE_ATTN", "auto")
+        # With block-scaled fp8 weights activations are rounded to e4m3 (per token and 128 features): half an ulp of bf16 in an attention output
+        # becomes a step of 6 to 12 % in a rounded one, and some per cent of the logits after a few layers (12 random steps of 13 sequences
+        # and 4 layers, the tensor-core kernel against the CUDA cores: 0 to 0.054 apart, the same steps in bf16 at most 0.015).  Such models
+        # keep the kernel and the chunks that their results were first computed with: 735 us instead of 700 for that step.
+        self.decode_keep_order = config is not None and config.quantization is not None
         self.fused_qkv_max_batch = int(os.environ.get("FORGE_FUSED_QKV_MAX", "32"))   # see models/qwen3.py
         self.sample_in_lm_head = os.environ.get("FORGE_LM_HEAD_SAMPLE", "1") != "0"
         # q/k-norm + RoPE + KV store in the qkv GEMM's epilogue (see qkv_rope_store_in_gemm): 174 instead of 201 launches per
@@ -308,13 +315,13 @@ class CudaOps(MixerOps, HybridOps):
             return out
         # graph-safe sizing: the longest context the block table can describe
         max_len = batch.table_width * k_cache.shape[2]
-        chunk, max_chunks = decode_chunking(B, k_cache.shape[1], k_cache.shape[2], max_len, H // k_cache.shape[1])
+        chunk, max_chunks = decode_chunking(B, k_cache.shape[1], k_cache.shape[2], max_len, 1 if self.decode_keep_order else H // k_cache.shape[1])
         part_o = part_ml = None
         if max_chunks > 1:
             part_o = torch.empty(B * H * max_chunks * D, dtype=torch.float32, device=q.device)
             part_ml = torch.empty(B * H * max_chunks * 2, dtype=torch.float32, device=q.device)
         self.C.decode_attention(q, k_cache, v_cache, batch.block_tables, batch.context_lens, out, part_o, part_ml,
-                                chunk, max_chunks, scale, self.status)
+                                chunk, max_chunks, scale, self.status, self.decode_keep_order)
         return out
 
     def _flat_ctas(self, num_heads, k_cache, from_raw_qkv: bool) -> int:
@@ -339,13 +346,14 @@ class CudaOps(MixerOps, HybridOps):
                                         out, self._flat_scratch, ctas, None, None, 0, 0, num_heads, scale, self.status)
             return out
         max_len = batch.table_width * k_cache.shape[2]
-        chunk, max_chunks = decode_chunking(B, k_cache.shape[1], k_cache.shape[2], max_len, num_heads // k_cache.shape[1])
+        chunk, max_chunks = decode_chunking(B, k_cache.shape[1], k_cache.shape[2], max_len, 1 if self.decode_keep_order else num_heads // k_cache.shape[1])
         part_o = part_ml = None
         if max_chunks > 1:
             part_o = torch.empty(B * num_heads * max_chunks * D, dtype=torch.float32, device=qkv.device)
             part_ml = torch.empty(B * num_heads * max_chunks * 2, dtype=torch.float32, device=qkv.device)
         self.C.decode_attention_qkv(qkv, q_weight, k_weight, eps, rope, k_cache, v_cache, batch.block_tables, batch.context_lens,
-                                    out, None, 0, part_o, part_ml, chunk, max_chunks, num_heads, scale, self.status)
+                                    out, None, 0, part_o, part_ml, chunk, max_chunks, num_heads, scale, self.status,
+                                    self.decode_keep_order)
         return out
 
     # ------------------------------------------------------------------ tensor-parallel exchange
