@@ -287,9 +287,9 @@ constexpr int kFewChunks = 24;
 
 __device__ __forceinline__ int decode_chunk_tokens(int len, const DecodeSplit& split) {
   const int units = (len + split.unit - 1) / split.unit;
-  int n = max((units + split.most - 1) / split.most, 1);           // units of a chunk
-  if (split.few)
-    while (units > n * max(kFewChunks, 12 * n)) ++n;
+  if (!split.few || units <= min(split.most, kFewChunks)) return split.unit;             // (not few: the longest context has `most` units)
+  int n = (units + split.most - 1) / split.most;                   // units of a chunk
+  while (units > n * max(kFewChunks, 12 * n)) ++n;
   return split.unit * n;
 }
 
