@@ -23,16 +23,8 @@
 
 namespace forge {
 
-constexpr int kCkTile = 64;
-constexpr int kCkBox = kCkTile * 128;                 // one TMA box: 64 token rows x 64 dims
-constexpr int kCkTileBytes = 2 * kCkBox;              // K (or V) of a tile: dims 0..63, then dims 64..127
 constexpr int kCkStages = 2;
 __host__ __device__ constexpr int ck_ctas_per_sm(int G) { return G > 4 ? 2 : 3; }
-
-// Shared-memory address of the 16-byte piece `piece` (0..15: eight dims each) of token row `r` of a swizzled tile.
-__device__ __forceinline__ uint32_t ck_addr(uint32_t tile, int r, int piece) {
-  return tile + (piece >> 3) * kCkBox + r * 128 + (((piece & 7) ^ (r & 7)) << 4);
-}
 
 // The parts of a weight: the upper 16 bits of p, of what is left, and of what is left then (at most 8 bits: exact).
 __device__ __forceinline__ float ck_upper(float p) { return __uint_as_float(__float_as_uint(p) & 0xFFFF0000u); }
@@ -100,7 +92,7 @@ __device__ __noinline__ void ck_repair_sums(float* o, const float* m, int heads,
 #pragma unroll
     for (int e = 0; e < 4; ++e) q[e] = __bfloat162float(q_rows[g * kD + 4 * lane + e]);
     const float m_use = m[g] == -INFINITY ? 0.f : m[g];
-    for (int tok0 = begin; tok0 < end; tok0 += kCkTile)
+    for (int tok0 = begin; tok0 < end; tok0 += kTcTile)
       for (int tok = tok0; tok < min(tok0 + 16, end); ++tok) {
         const int blk = table[tok / block_size];
         const size_t off = ((static_cast<size_t>(blk >= 0 && blk < num_blocks ? blk : 0) * nkv + kvh) * block_size + tok % block_size) * kD + 4 * lane;
@@ -128,7 +120,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
   static_assert(G <= 8, "the heads of a group fill the first eight rows of the query tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* s_acc = reinterpret_cast<float*>(smem + kCkStages * 2 * kCkTileBytes);          // merge area
+  float* s_acc = reinterpret_cast<float*>(smem + kCkStages * 2 * kTcTileBytes);          // merge area
   __nv_bfloat16* s_q = reinterpret_cast<__nv_bfloat16*>(s_acc + decode_merge_floats(G)); // [G][128]
   uint4* s_new = reinterpret_cast<uint4*>(s_q + G * kD); // the newest token: 16 pieces of its key, 16 of its value
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(s_new + 32);
@@ -157,7 +149,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
     for (int item = blockIdx.x; ok && chunk_item(context_lens, B, nkv, split, cap, direct != 0, item, status, it); item += gridDim.x) {
       if (lane == 0) {
         const int end = min(it.len, (it.c + 1) * it.chunk);
-        for (int tok = it.c * it.chunk; tok < end; tok += kCkTile, ++n) {
+        for (int tok = it.c * it.chunk; tok < end; tok += kTcTile, ++n) {
           const int s = n % kCkStages;
           int blk = block_tables[static_cast<size_t>(it.b) * table_width + tok / block_size];
           if (blk < 0 || blk >= num_blocks) {
@@ -167,12 +159,12 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
           const int row = (blk * nkv + it.kvh) * block_size + tok % block_size;
           ok = mbar_wait(&empty_bar[s], ((n / kCkStages) & 1) ^ 1, status);
           if (!ok) break;
-          uint8_t* stg = smem + s * 2 * kCkTileBytes;
-          mbar_expect_tx(&full_bar[s], 2 * kCkTileBytes);
+          uint8_t* stg = smem + s * 2 * kTcTileBytes;
+          mbar_expect_tx(&full_bar[s], 2 * kTcTileBytes);
           tma_load_2d(stg, &tm_k, &full_bar[s], 0, row);
-          tma_load_2d(stg + kCkBox, &tm_k, &full_bar[s], 64, row);
-          tma_load_2d(stg + kCkTileBytes, &tm_v, &full_bar[s], 0, row);
-          tma_load_2d(stg + kCkTileBytes + kCkBox, &tm_v, &full_bar[s], 64, row);
+          tma_load_2d(stg + kTcBoxBytes, &tm_k, &full_bar[s], 64, row);
+          tma_load_2d(stg + kTcTileBytes, &tm_v, &full_bar[s], 0, row);
+          tma_load_2d(stg + kTcTileBytes + kTcBoxBytes, &tm_v, &full_bar[s], 64, row);
         }
       }
       ok = __all_sync(0xffffffffu, ok);
@@ -195,7 +187,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
     const int qh0 = it.kvh * G, begin = it.c * it.chunk, end = min(it.len, begin + it.chunk);
     if (begin >= end) continue;                         // uniform for the consumers
     // the newest token (position len - 1) is not in the cache yet: the warp that owns its row of its tile prepares it now
-    const int newest = it.len - 1, row_new = newest % kCkTile;
+    const int newest = it.len - 1, row_new = newest % kTcTile;
     const bool owner = fuse.qkv != nullptr && newest >= begin && newest < end && warp == row_new / 16;
     uint32_t qa[8][2];                                  // rows 0..G-1 = the heads of the group, the others zero (G = 4: again the heads); 8 steps of 16 dims
     if (fuse.qkv != nullptr) {
@@ -232,18 +224,18 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
     float o[16][4];                                     // [..][0, 1]: sums of hi V (lo_row: of lo V), [2, 3]: of mid V (and of lo V), same head and dims
 #pragma unroll
     for (int nb = 0; nb < 16; ++nb) o[nb][0] = o[nb][1] = o[nb][2] = o[nb][3] = 0.f;
-    for (int tok0 = begin; tok0 < end; tok0 += kCkTile, ++n) {
+    for (int tok0 = begin; tok0 < end; tok0 += kTcTile, ++n) {
       const int s = n % kCkStages;
       ok = ok && mbar_wait(&full_bar[s], (n / kCkStages) & 1, status);
-      uint8_t* stg = smem + s * 2 * kCkTileBytes;
-      const uint32_t Ks = smem_u32(stg), Vs = Ks + kCkTileBytes;
-      if (owner && newest - tok0 < kCkTile) {           // its tile: the row is put in place, and into the cache for later steps
+      uint8_t* stg = smem + s * 2 * kTcTileBytes;
+      const uint32_t Ks = smem_u32(stg), Vs = Ks + kTcTileBytes;
+      if (owner && newest - tok0 < kTcTile) {           // its tile: the row is put in place, and into the cache for later steps
         int blk = block_tables[static_cast<size_t>(it.b) * table_width + newest / block_size];
         const bool to_cache = blk >= 0 && blk < num_blocks;
         if (!to_cache) blk = 0;
         const size_t off = ((static_cast<size_t>(blk) * nkv + it.kvh) * block_size + newest % block_size) * kD;
         const uint4 piece = s_new[lane];
-        *reinterpret_cast<uint4*>(stg + (ck_addr(lane < 16 ? Ks : Vs, row_new, lane & 15) - Ks)) = piece;
+        *reinterpret_cast<uint4*>(stg + (tc_tile_addr(lane < 16 ? Ks : Vs, row_new, lane & 15) - Ks)) = piece;
         if (to_cache) *reinterpret_cast<uint4*>((lane < 16 ? k_cache : v_cache) + off + 8 * (lane & 15)) = piece;
         fence_proxy_async_smem();                       // a later copy into this stage comes after these writes
         __syncwarp();
@@ -255,7 +247,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
         uint32_t kb[4];
-        ldsm_x4(ck_addr(Ks, r0 + (mat >> 1) * 8 + mrow, 2 * kk + (mat & 1)), kb);
+        ldsm_x4(tc_tile_addr(Ks, r0 + (mat >> 1) * 8 + mrow, 2 * kk + (mat & 1)), kb);
         const uint32_t a[4] = {qa[kk][0], 0u, qa[kk][1], 0u};
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -309,7 +301,7 @@ __global__ void __launch_bounds__(kDecThreads, ck_ctas_per_sm(G)) decode_attn_ch
 #pragma unroll
       for (int dd = 0; dd < 8; ++dd) {
         uint32_t vb[4];
-        ldsm_x4_trans(ck_addr(Vs, r0 + (mat & 1) * 8 + mrow, 2 * dd + (mat >> 1)), vb);
+        ldsm_x4_trans(tc_tile_addr(Vs, r0 + (mat & 1) * 8 + mrow, 2 * dd + (mat >> 1)), vb);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           float c[4] = {0.f, 0.f, 0.f, 0.f};
@@ -381,13 +373,13 @@ template <int G>
 static int launch_chunks(const void* q, const void* kc, const void* vc, const int* bt, const int* lens, void* out, float* part_o, float* part_ml, int B,
                          int nq, int nkv, int block_size, int table_width, int num_blocks, const DecodeSplit& split, int max_chunks, float scale_log2, unsigned* status,
                          cudaStream_t stream, const DecodeFuse& fuse) {
-  constexpr int smem = kCkStages * 2 * kCkTileBytes + decode_merge_floats(G) * 4 + G * kD * 2 + 512 + 2 * kCkStages * 8 + 1024;
+  constexpr int smem = kCkStages * 2 * kTcTileBytes + decode_merge_floats(G) * 4 + G * kD * 2 + 512 + 2 * kCkStages * 8 + 1024;
   static_assert(ck_ctas_per_sm(G) * (smem + 1024) <= 228 * 1024, "CTAs per SM");
   auto kern = decode_attn_chunk_kernel<G>;
   FORGE_ENSURE_DYN_SMEM(kern, smem);
   CUtensorMap tm_k, tm_v;
   const uint64_t rows = static_cast<uint64_t>(num_blocks) * nkv * block_size;
-  if (forge_make_tmap_2d(&tm_k, kc, rows, kD, kD, kCkTile, 2) != 0 || forge_make_tmap_2d(&tm_v, vc, rows, kD, kD, kCkTile, 2) != 0) return -2;
+  if (forge_make_tmap_2d(&tm_k, kc, rows, kD, kD, kTcTile, 2) != 0 || forge_make_tmap_2d(&tm_v, vc, rows, kD, kD, kTcTile, 2) != 0) return -2;
   // up to two waves of CTAs: one per item, dead ones included (they end at once, and no list is walked); else the live ones over one wave
   const long long most = static_cast<long long>(B) * nkv * split.most;
   const int wave = ck_ctas_per_sm(G) * device_sm_count();

@@ -10,9 +10,10 @@
 //   * four consumer warps each own a quarter of every tile and keep their own online-softmax state,
 //     so the main loop has no CTA-wide barrier; the q heads that share a KV head are processed together
 //     (each K/V byte is read from shared memory once per group);
-//   * the context is cut into fixed-size chunks (grid.z); each CTA writes either the final output (one
-//     chunk) or a normalised partial plus (max, sum) that a small second kernel merges.  Lengths are read
-//     on the device, so the launch is CUDA-graph safe: the grid depends only on the batch bucket.
+//   * few sequences: the context is cut into chunks (grid.z; their size follows from the length, DecodeSplit); each CTA
+//     writes either the final output (one chunk) or a normalised partial plus (max, sum) that a small second kernel
+//     merges.  Many: all tiles of the step are dealt out equally (the flat partition below).  Lengths are read on the
+//     device, so the launch is CUDA-graph safe: the grid depends only on the batch bucket.
 //
 // head_dim is 128 (all Qwen3 sizes).  Scores use exp2 with the scale folded into q.
 #include <algorithm>
@@ -20,6 +21,7 @@
 
 #include "../include/decode_common.cuh"
 #include "../include/launch.cuh"
+#include "../include/mma_sync.cuh"
 #include "../include/ptx.cuh"
 
 namespace forge {
@@ -629,24 +631,11 @@ static int launch_decode_flat(const void* q, const void* kc, const void* vc, con
 // kernel at 0.55 of copy bandwidth; one 256-byte bulk copy per row with a padded pitch ran at 0.17.)
 // Groups of up to 5 heads leave room for two CTAs per SM (three stages each); 8 heads take one CTA with six stages.
 // =========================================================================================================
-constexpr int kTcTile = 64;
-constexpr int kTcBoxBytes = kTcTile * 128;            // one TMA box: 64 token rows x 64 dims
-constexpr int kTcTileBytes = 2 * kTcBoxBytes;         // K (or V) of a tile: dims 0..63, then dims 64..127
 extern "C" int forge_make_tmap_2d(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
                                   int elem_bytes);
-// Shared-memory address of the 16-byte chunk `chunk` (0..15: eight dims each) of token row `r` of a swizzled tile.
-__device__ __forceinline__ uint32_t tc_chunk_addr(uint32_t tile, int r, int chunk) {
-  return tile + (chunk >> 3) * kTcBoxBytes + r * 128 + (((chunk & 7) ^ (r & 7)) << 4);
-}
 __host__ __device__ constexpr int tc_ctas_per_sm(int G) { return G > 5 ? 1 : 2; }
 __host__ __device__ constexpr int tc_stages(int G) { return G > 5 ? 6 : 3; }
 
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
 // D (16 x 8, fp32) += A (16 x 16, bf16, rows 8..15 zero: a1 = a3 = 0) * B (16 x 8, bf16)
 __device__ __forceinline__ void mma_rows8(float (&c)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -798,7 +787,7 @@ __global__ void __launch_bounds__(kDecThreads, tc_ctas_per_sm(G)) decode_attn_fl
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk) {
         uint32_t kb[4];
-        ldmatrix_x4(kb, tc_chunk_addr(Ks, r0 + (mat >> 1) * 8 + mrow, 2 * kk + (mat & 1)));
+        ldsm_x4(tc_tile_addr(Ks, r0 + (mat >> 1) * 8 + mrow, 2 * kk + (mat & 1)), kb);
         mma_rows8(sc[0], qa[kk][0], qa[kk][1], kb[0], kb[1]);
         mma_rows8(sc[1], qa[kk][0], qa[kk][1], kb[2], kb[3]);
       }
@@ -835,7 +824,7 @@ __global__ void __launch_bounds__(kDecThreads, tc_ctas_per_sm(G)) decode_attn_fl
 #pragma unroll
       for (int dd = 0; dd < 8; ++dd) {
         uint32_t vb[4];
-        ldmatrix_x4_trans(vb, tc_chunk_addr(Vs, r0 + (mat & 1) * 8 + mrow, 2 * dd + (mat >> 1)));
+        ldsm_x4_trans(tc_tile_addr(Vs, r0 + (mat & 1) * 8 + mrow, 2 * dd + (mat >> 1)), vb);
         mma_rows8(o[2 * dd], pa0, pa2, vb[0], vb[1]);
         mma_rows8(o[2 * dd + 1], pa0, pa2, vb[2], vb[3]);
       }

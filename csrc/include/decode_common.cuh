@@ -10,6 +10,15 @@ constexpr int kD = 128;
 constexpr int kDecStages = 3;
 constexpr int kDecThreads = 160;   // 4 consumer warps + 1 producer warp
 
+// A tile of the tensor-core kernels: 64 tokens of K (or of V) as two TMA boxes with the 128-byte swizzle.
+constexpr int kTcTile = 64;
+constexpr int kTcBoxBytes = kTcTile * 128;            // one box: 64 token rows x 64 dims
+constexpr int kTcTileBytes = 2 * kTcBoxBytes;         // dims 0..63, then dims 64..127
+// Shared-memory address of the 16-byte piece `piece` (0..15: eight dims each) of token row `r` of a tile.
+__device__ __forceinline__ uint32_t tc_tile_addr(uint32_t tile, int r, int piece) {
+  return tile + (piece >> 3) * kTcBoxBytes + r * 128 + (((piece & 7) ^ (r & 7)) << 4);
+}
+
 // q heads that share a KV head are processed together in slices of G heads (each K/V byte is read from shared memory
 // once per slice, and streamed from the cache once per slice): the largest supported G that divides the group.  G <= 4
 // leaves room for two CTAs per SM; G = 5 (Qwen3-14B: 40 / 8 heads) takes the registers of a whole SM but reads the cache
