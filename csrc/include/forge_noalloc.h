@@ -21,7 +21,8 @@
  * Tensors (all device pointers, bf16 unless noted):
  *   q [B, nq, 128]; k_cache, v_cache [num_blocks, nkv, block_size, 128]; block_tables int32 [B, table_width];
  *   context_lens int32 [B]; out [B, nq * 128]; status: optional device word that collects error bits.
- *   chunk: tokens per context slice, a multiple of min(block_size, 64); max_chunks * chunk >= longest context.
+ *   chunk: tokens of the smallest context slice, a multiple of min(block_size, 64) (with few sequences the kernel may
+ *   make slices a multiple of it); max_chunks * chunk >= longest context.
  * Returns 0 on success, a negative code otherwise (see forge_decode_attention_noalloc_strerror).
  */
 #pragma once
