@@ -3,7 +3,8 @@
     python -m tinyllmforge_b200.utils.kernel_case <case> [--iters N] [--lib] [--peaks FILE]
 
 Cases: decode_attention (64 sequences x 2048 tokens, 16 / 8 heads), decode_attention_g4 (256 x 800, 32 / 8 heads: Qwen3-8B),
-decode_attention_g8 (64 x 2304, 64 / 8 heads: Qwen3-32B), prefill_attention, gemm_decode, gemm_decode_split, gemm_prefill,
+decode_attention_g8 (64 x 2304, 64 / 8 heads: Qwen3-32B), decode_attention_few (24 x 3000, 32 / 8 heads: context chunks), prefill_attention,
+qkv_prompt (3777 x 6144 x 4096 with norm, rotation and cache write in the epilogue), gemm_decode, gemm_decode_split, gemm_prefill,
 gemm_prefill_8b (8192 x 6144 x 4096), gemm_silu, gemm_fp8 (256 x 6144 x 4096, block-scaled e4m3 weights), gemm_residual (o_proj-like GEMM with the residual add + sums of squares
 epilogue), gemm_scaled (qkv-like GEMM with the folded-norm row scale), gemm_decode_8b_down (256 x 4096 x 12288 with the residual
 epilogue: K split over CTA pairs + the reduce kernel), lm_head_sample (LM head + sampling in one kernel),
@@ -61,9 +62,9 @@ def _paged(B, ctx, nq, nkv, bs, q_len=1):
 
 def build(case: str, ops, lib: bool = False):
     """Returns (callable, bytes moved per launch, flops per launch)."""
-    if case in ("decode_attention", "decode_attention_g4", "decode_attention_g8"):
+    if case in ("decode_attention", "decode_attention_g4", "decode_attention_g8", "decode_attention_few"):
         B, ctx, nq, nkv = {"decode_attention": (64, 2048, 16, 8), "decode_attention_g4": (256, 800, 32, 8),
-                           "decode_attention_g8": (64, 2304, 64, 8)}[case]
+                           "decode_attention_g8": (64, 2304, 64, 8), "decode_attention_few": (24, 3000, 32, 8)}[case]
         ctx_alloc = -(-ctx // 256) * 256
         q, kc, vc, b = _paged(B, ctx_alloc, nq, nkv, 256)
         b.context_lens.fill_(ctx)
@@ -158,6 +159,18 @@ def build(case: str, ops, lib: bool = False):
         kc = torch.zeros(T // bs, nkv, bs, 128, device="cuda", dtype=BF)
         vc = torch.zeros_like(kc)
         return (lambda: ops.qk_norm_rope_store(qkv, w, w, 1e-6, table, pos, slots, kc, vc, nq, nkv, 128)), 2 * T * (nq + 2 * nkv) * 128 * 2, 0
+    if case == "qkv_prompt" and not lib:
+        from ..ops import ref
+        T, K, nq, nkv, bs = 3777, 4096, 32, 8, 256
+        w, x = torch.randn((nq + 2 * nkv) * 128, K, device="cuda", dtype=BF) * 0.02, torch.randn(T, K, device="cuda", dtype=BF)
+        norm = torch.ones(128, device="cuda", dtype=BF)
+        ssq = (x.float() ** 2).view(T, K // 128, 128).sum(-1).contiguous()
+        table = ref.rope_table(4096, 128, 1e6, "cuda")
+        pos = torch.arange(T, dtype=torch.int32, device="cuda")
+        kc = torch.zeros(-(-T // bs), nkv, bs, 128, device="cuda", dtype=BF)
+        vc = torch.zeros_like(kc)
+        return ((lambda: ops.linear_qkv_rope_store(x, w, ssq, 1e-6, norm, norm, 1e-6, table, pos, pos, kc, vc, nq, nkv)),
+                (w.numel() + x.numel() + T * w.shape[0]) * 2, 2 * T * w.numel())
     if case == "sampler":
         logits = torch.randn(256, 151936, device="cuda", dtype=BF)
         temps = torch.full((256,), 0.6, device="cuda")
