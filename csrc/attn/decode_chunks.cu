@@ -10,10 +10,12 @@
 // finished here, others leave partials for the merge kernel.
 //
 // What bounds it is latency (length -> block table -> keys -> scores -> sums), and from about ten sequences the stream of the cache: three
-// CTAs per SM with 64 KB on their way each.  The dot products on the CUDA cores, which this replaces for cache blocks of 64 tokens and more,
-// took longer than the stream: a tile of 64 tokens of four heads needs 64 K multiply-adds and 2500 shuffles in a warp.
-// Measured with the merge, 32 / 8 heads (CUDA cores): 1 x 3001 tokens 24.2 -> 13.3 us, 8 x 200 .. 2000: 21.0 -> 17.8, 13: 31.7 -> 22.4, 24: 54.5 -> 39.8;
-// 64 / 8 heads, 24 x 200 .. 2000: 91 -> 36 us.  The error against 64 bits is the same (1.9e-3, the rounding of the result to bf16).
+// CTAs per SM (two for groups of more than four, whose third part of the weights takes registers) with 64 KB on their way each.  The dot products
+// on the CUDA cores, which this replaces for cache blocks of 64 tokens and more, took longer than the stream: a tile of 64 tokens of four heads needs
+// 64 K multiply-adds and 2500 shuffles in a warp.
+// Measured with the merge (CUDA cores -> here), 32 / 8 heads: 1 x 3001 tokens 18.6 -> 11.1 us, 13 x 200 .. 2000 34.5 -> 26.8; 64 / 8 heads: 23.1 -> 11.4,
+// 58 -> 33.9.  Error of the fp32 partials against 64 bits (CUDA cores -> here): 3001 tokens 8.2e-8 -> 6.3e-8, values without a common direction
+// 2.1e-7 -> 1.4e-7, chunks of 1536 tokens 3.8e-7 -> 1.7e-7; of the bf16 result 1.67e-3 both.
 #include <algorithm>
 
 #include "../include/decode_common.cuh"

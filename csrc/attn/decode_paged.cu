@@ -293,7 +293,7 @@ static int decode_chunked_impl(const void* q, const void* kc, const void* vc, co
   const DecodeSplit split = {chunk, few ? std::min(max_chunks, std::max(kFewChunks, device_sm_count() / (B * nkv))) : max_chunks, few};
   // Groups of 4 to 8 heads, cache blocks of 64 tokens and more: on the tensor cores (decode_chunks.cu).  With two heads per
   // KV head the CUDA cores keep up with the stream and their kernel starts faster (2 sequences 12.0 us against 13.8, 40: 44 against 53); with four
-  // they do not (13 sequences: 31.7 against 22.4).
+  // they do not (13 sequences: 34.5 against 26.8).
   if (tile == 64 && group >= 4 && group <= 8 && keep_order == 0) {
     const int rc = launch_decode_chunks(q, kc, vc, bt, lens, out, part_o, part_ml, B, nq, nkv, block_size, table_width, num_blocks, split, max_chunks, sl2,
                                         status, stream, fuse);

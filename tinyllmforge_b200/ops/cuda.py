@@ -44,8 +44,8 @@ def decode_chunking(batch: int, num_kv_heads: int, block_size: int, max_len: int
     Small batches split the context finely so that every SM gets work; large batches keep chunks long so
     that the partial-merge traffic stays negligible.  Depends only on shapes known at graph-capture time.
     The kernel may make chunks a multiple of this long (few sequences); the number of chunks is what scratch is sized for.
-    Groups of 4 to 8 query heads run on the tensor cores with a fixed cost per chunk, which longer chunks share: measured with 32 / 8
-    heads and 200..2000 tokens, chunks of 128 / 256 / 512: 4 sequences 14.5 / 14.8 / 16.7 us, 8: 22.9 / 17.2 / 19.3, 13: 35.2 / 27.6 / 22.4, 24: 63 / 47 / 40;
+    Groups of 4 to 8 query heads run on the tensor cores with a fixed cost per chunk, which longer chunks share: measured (before their
+    weights had 24 bits) with 32 / 8 heads and 200..2000 tokens, chunks of 128 / 256 / 512: 4 sequences 14.5 / 14.8 / 16.7 us, 8: 22.9 / 17.2 / 19.3, 13: 35.2 / 27.6 / 22.4, 24: 63 / 47 / 40;
     with 8 / 1 heads these sizes give 10.4 us for 8 sequences, 11.5 for 13, 9.9 for 24, 13.1 for 40 (CUDA cores and their sizes: 14.6, 21.3, 16.4, 18.3)."""
     tile = min(block_size, 64)
     ctas = batch * num_kv_heads
